@@ -1441,6 +1441,477 @@ __global__ void __launch_bounds__(kPThreads, MODE == 1 ? 1 : 2) k_pcg_persistent
   if (cta == 0 && threadIdx.x == 0 && *(volatile int*)&c->bar_error) c->done = kDoneBarrierTimeout;
 }
 
+// ---------------------------------------------------- one-cluster FP64 CG ---
+// Small FP64 CSR systems.  A grid-wide persistent launch pays three grid
+// barriers and a chain of dependent L2 loads per iteration whatever the size.
+// Here one thread-block cluster holds the whole system in its CTAs' shared
+// memory for the length of the solve: matrix values with 16-bit column codes
+// and, of the direction p, the window of columns that the CTA's rows touch.
+// x, r and the preconditioner of a row stay in its thread's registers, so an
+// iteration touches no global memory.
+//
+// What bounds it is FP64 latency: a warp's FP64 instruction holds its
+// sub-partition's unit for 64 cycles, dependent or not, predicated off or not.
+// So
+//  - a CTA picks the lanes per row (1, 2, 4, 8) that need the fewest FP64
+//    instructions in sequence over its four sub-partitions;
+//  - sums over lanes run on the integer pipe (warp_sum_fixed: 230 cycles
+//    against 540 for the FP64 tree), as do tests for zero and finite values;
+//  - everything that crosses the cluster (every warp's share of a dot product,
+//    the new p of a row for the windows that hold it) goes as st.async words
+//    that complete on the receiver's mbarrier: one hop, and no cluster barrier
+//    within an iteration;
+//  - 1 / r.z, wanted by the next beta, is formed by a warp that would wait.
+//
+// Rows are split over the CTAs by stored entries.  Within a CTA they are taken
+// in descending length, a warp storing its entries step-major (entry j of a
+// row on lane j % L): reads of the matrix are free of bank conflicts and little
+// padding is stored.  Every CTA sums the same shares in the same order, so
+// all take the same decisions and results are deterministic.  A system that
+// does not fit (shared memory, rows per CTA) is declined before the first
+// iteration and left to the grid-wide kernel.
+constexpr int kClMax = 16;        // CTAs per cluster (non-portable size; 8 where 16 cannot be placed)
+constexpr int kClThreads = 256;
+constexpr int kClWarps = kClThreads / 32;
+constexpr int kClOwn = 4;            // rows of a thread in the vector phases
+constexpr int kClRows = kClOwn * kClThreads;
+constexpr int kClSmem = 222 * 1024;  // dynamic shared memory per CTA
+constexpr int kClWide = 256;         // CTAs with more rows take one lane per row
+constexpr int kClBlocks = kClWide * 8 / 32;  // warp blocks of a CTA at most
+constexpr int kClNoFit = 100;        // ctrl->done: left to the grid-wide kernel
+
+struct ClusterParams {
+  int64_t n;
+  const int64_t* row_ptr;
+  const int32_t* col;
+  const double* val;
+  const double* dinv;
+  const double* b;
+  double* x;
+  Ctrl* ctrl;
+  double rtol2;
+  long long max_iter;
+};
+
+__device__ __forceinline__ uint32_t cl_map(uint32_t addr, uint32_t rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ int cl_ld(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+// v to address dst of CTA `rank`, completing 8 bytes on that CTA's barrier.
+__device__ __forceinline__ void cl_send(uint32_t dst, uint32_t bar, uint32_t rank, double v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(cl_map(dst, rank)),
+               "l"(__double_as_longlong(v)), "r"(cl_map(bar, rank))
+               : "memory");
+}
+__device__ __forceinline__ void cl_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool cl_wait(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (clock64() - t0 > kMbarSpin) return false;
+  }
+}
+
+// Sums of K doubles per lane on the integer pipe, the same values in every
+// lane: each is aligned to its largest exponent as a 58-bit integer (five
+// bits below an FP64 mantissa, rounded to nearest), added exactly in three
+// redux words and rounded to FP64 once.  The error is at most 32 half units
+// of 2^-58 of the largest value plus that rounding, no more than five FP64
+// additions leave.  Exponents at either end of the range (and NaN,
+// infinities) take the FP64 tree.
+template <int K>
+__device__ __forceinline__ void sum_fixed(double (&v)[K]) {
+  int ex[K], e[K];
+  bool plain = true;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    ex[k] = (__double2hiint(v[k]) >> 20) & 0x7ff;
+    e[k] = (int)__reduce_max_sync(0xffffffffu, (unsigned)ex[k]);
+    plain = plain && e[k] >= 128 && e[k] <= 1990;
+  }
+  if (!plain) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      v[k] = __any_sync(0xffffffffu, (__double_as_longlong(v[k]) << 1) != 0) ? warp_sum(v[k]) : 0.0;
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const long long bits = __double_as_longlong(v[k]);
+    const int sh = min(e[k] - ex[k], 62);
+    unsigned long long m = ((unsigned long long)(bits & 0xfffffffffffffLL) | (1ull << 52)) << 5;
+    m = ex[k] == 0 ? 0ull : (m + ((1ull << sh) >> 1)) >> sh;
+    const long long f = bits < 0 ? -(long long)m : (long long)m;
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)f & 0x3fffffu);
+    const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 22) & 0x3fffffu);
+    const int hi = __reduce_add_sync(0xffffffffu, (int)(f >> 44));
+    const long long t = ((long long)hi << 44) + ((long long)mid << 22) + (long long)lo;
+    v[k] = t == 0 ? 0.0 : __longlong_as_double(__double_as_longlong((double)t) + ((long long)(e[k] - 1080) << 52));
+  }
+}
+
+// Kept out of line: an iteration calls them five times, and straight-line code
+// that runs once an iteration is fetched more slowly than it executes.
+__device__ __noinline__ double warp_sum_fixed(double a) {
+  double v[1] = {a};
+  sum_fixed<1>(v);
+  return v[0];
+}
+__device__ __noinline__ double2 warp_sum_fixed2(double a, double b) {
+  double v[2] = {a, b};
+  sum_fixed<2>(v);
+  return make_double2(v[0], v[1]);
+}
+
+// isfinite and == 0 by the bits: a comparison costs an FP64 instruction.
+__device__ __forceinline__ bool finite_bits(double v) { return ((__double2hiint(v) >> 20) & 0x7ff) != 0x7ff; }
+__device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
+
+// Sum of the n shares that the cluster's warps sent, on one warp.
+__device__ __forceinline__ double cl_total(const double* part, int n) {
+  const int lane = threadIdx.x & 31;
+  double s = lane < n ? part[lane] : 0.0;
+  for (int i = 32; i < n; i += 32) s += i + lane < n ? part[i + lane] : 0.0;
+  return warp_sum_fixed(s);
+}
+
+__global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) {
+  __shared__ int64_t lo_s[kClMax + 1];           // first row of every CTA
+  __shared__ int base_s[kClBlocks + 1];          // first slot-row of every warp block
+  __shared__ double part[3][kClMax * kClWarps];  // every warp's share of p.q, r.z and r.r
+  __shared__ __align__(8) unsigned long long bar_s[3];
+  __shared__ double sh_scalar, sh_rz, sh_inv;
+  __shared__ int sh_done[2], fit_s, fail_s, lanes_s, cost_s[4], steps_s[4];
+  __shared__ int info_s[3], all_s[kClMax][3];  // first and past-last column of the window, warps with blocks
+  extern __shared__ __align__(128) unsigned char dyn_smem[];
+  constexpr int T = kClThreads, W = kClWarps;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t rank, NC;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(NC));
+  const uint32_t bar_a = smem_u32(&bar_s[0]), bar_b = smem_u32(&bar_s[1]), bar_p = smem_u32(&bar_s[2]);
+
+  // ---- rows of every CTA: equal shares of the stored entries
+  if (tid <= (int)NC) {
+    const int64_t total = P.row_ptr[P.n];
+    lo_s[tid] = tid == (int)NC ? P.n : lower_bound_i64(P.row_ptr, P.n, total * tid / NC);
+  }
+  if (tid == 0) {
+    for (int k = 0; k < 3; ++k) mbar_init(smem_u32(&bar_s[k]));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const int64_t row_lo = lo_s[rank];
+  const bool small = lo_s[rank + 1] - row_lo <= kClRows;
+  const int R = small ? (int)(lo_s[rank + 1] - row_lo) : 0;
+  // the window of columns (n is at most kClMax * kClRows)
+  if (tid == 0) {
+    info_s[0] = (int)row_lo;
+    info_s[1] = (int)row_lo + R;
+  }
+  __syncthreads();
+  {
+    int first = (int)row_lo, last = (int)row_lo + R - 1;
+    const int64_t e1 = P.row_ptr[row_lo + R];
+#pragma unroll 4
+    for (int64_t i = P.row_ptr[row_lo] + tid; i < e1; i += T) {
+      const int c = P.col[i];
+      first = min(first, c);
+      last = max(last, c);
+    }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+      atomicMin(&info_s[0], first);
+      atomicMax(&info_s[1], last + 1);
+    }
+  }
+  __syncthreads();
+  const int w0 = info_s[0], wn = info_s[1] - w0, own = (int)row_lo - w0;
+  double* pw_s = reinterpret_cast<double*>(dyn_smem);  // the window of p, at the same address in every CTA
+  double* q_s = pw_s + wn;
+  double* val_s = q_s + R;
+  int* len_s = reinterpret_cast<int*>(pw_s);  // set-up only: row lengths
+  int* perm_s = reinterpret_cast<int*>(q_s);  // set-up only: rows by descending length
+  const int fixed = (R + wn) * (int)sizeof(double) + R * (int)sizeof(uint16_t);
+  const int max_steps = (kClSmem - fixed) / (32 * 10);
+  const bool room = small && max_steps > 0;
+  const int Rs = room ? R : 0;  // rows of the set-up
+  for (int a = tid; a < Rs; a += T)
+    len_s[a] = (int)min((int64_t)(1 << 20), P.row_ptr[row_lo + a + 1] - P.row_ptr[row_lo + a]);
+  __syncthreads();
+  for (int a = tid; a < Rs; a += T) {
+    const int len = len_s[a];
+    int place = 0;
+    for (int i = 0; i < R; ++i) place += len_s[i] > len || (len_s[i] == len && i < a);
+    perm_s[place] = a;
+  }
+  __syncthreads();
+  // lanes per row: the fewest FP64 instructions in sequence (a block's steps,
+  // its lane sums and its p.q product) on the busiest of four sub-partitions
+  // among those that fit; the longest row of a block is its first
+  if (tid < 4) {
+    const int L = 1 << tid, rpb = 32 >> tid;
+    int total = 0, steps = 0, longest = 0;
+    if (tid == 0 || Rs <= kClWide)
+      for (int k = 0; k * rpb < Rs && steps <= max_steps; ++k) {
+        const int st = (len_s[perm_s[k * rpb]] + L - 1) / L;
+        const int ops = 2 * (st + 1) + 3 * tid;  // a shuffled addition costs half as much again
+        steps += st;
+        total += ops;
+        longest = max(longest, ops);
+      }
+    else
+      steps = max_steps + 1;
+    cost_s[tid] = max((total + 3) / 4, longest);
+    steps_s[tid] = steps;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int best = -1;
+    for (int k = 0; k < 4; ++k)
+      if (steps_s[k] <= max_steps && (best < 0 || cost_s[k] < cost_s[best])) best = k;
+    lanes_s = best;
+    fit_s = room && best >= 0;
+    fail_s = 0;
+    if (best >= 0) info_s[2] = min(W, (R + (32 >> best) - 1) / (32 >> best));
+  }
+  cl_sync();
+  if (tid < 3 * (int)NC) all_s[tid / 3][tid % 3] = cl_ld(cl_map(smem_u32(&info_s[tid % 3]), tid / 3));
+  int fits = 1;
+  for (uint32_t c = 0; c < NC; ++c) fits &= cl_ld(cl_map(smem_u32(&fit_s), c));
+  if (!fits) {
+    cl_sync();  // no CTA leaves while another reads its flag
+    if (rank == 0 && tid == 0) P.ctrl->done = kClNoFit;
+    return;
+  }
+  const int lsh = lanes_s, L = 1 << lsh, rpb = 32 >> lsh;
+  const int nb = (R + rpb - 1) / rpb;
+  if (tid == 0) {
+    int at = 0;
+    for (int k = 0; k < nb; ++k) {
+      base_s[k] = at;
+      at += (len_s[perm_s[k * rpb]] + L - 1) >> lsh;
+    }
+    base_s[nb] = at;
+  }
+  __syncthreads();
+  uint16_t* code_s = reinterpret_cast<uint16_t*>(val_s + (size_t)base_s[nb] * 32);
+  uint16_t* row_s = code_s + (size_t)base_s[nb] * 32;  // rows by descending length
+  for (int a = tid; a < R; a += T) row_s[a] = (uint16_t)perm_s[a];
+  // where this CTA's shares go, and how many there are: the warps with blocks
+  // share p.q, the warps with rows r.z and r.r
+  int at_a = 0, at_b = 0, n_a = 0, n_b = 0;
+  for (uint32_t c = 0; c < NC; ++c) {
+    const int wa = all_s[c][2], wb = min(W, (int)(lo_s[c + 1] - lo_s[c] + 31) / 32);
+    if (c < rank) {
+      at_a += wa;
+      at_b += wb;
+    }
+    n_a += wa;
+    n_b += wb;
+  }
+
+  // ---- matrix into shared memory; padding is a zero times the window's first p
+  for (int k = warp; k < nb; k += W) {
+    const int slot = k * rpb + (lane >> lsh);
+    const int row = slot < R ? perm_s[slot] : 0;
+    const int64_t rs = P.row_ptr[row_lo + row];
+    const int len = slot < R ? len_s[row] : 0;
+    const int b0 = base_s[k], steps = base_s[k + 1] - b0;
+#pragma unroll 4
+    for (int j = 0; j < steps; ++j) {
+      const int at = (j << lsh) + (lane & (L - 1));
+      const bool in = at < len;
+      val_s[(size_t)(b0 + j) * 32 + lane] = in ? P.val[rs + at] : 0.0;
+      code_s[(size_t)(b0 + j) * 32 + lane] = (uint16_t)(in ? P.col[rs + at] - w0 : 0);
+    }
+  }
+  // len_s and perm_s end here, in every CTA: the windows may be written
+  cl_sync();
+
+  // ---- start from x = 0
+  // rows tid + u T, u < nu (the same nu on every lane; a branch, not a
+  // predicate, keeps the FP64 unit free where a warp has no rows left)
+  const int nu = (R - warp * 32 + T - 1) / T;
+  double x[kClOwn], r[kClOwn], mi[kClOwn], z[kClOwn], p[kClOwn];
+  const uint32_t pw_base = smem_u32(pw_s);
+  uint32_t phase_p = 0;
+  // p of this CTA's rows into every window that holds them (a run of rows for
+  // each CTA, one warp sending it); returns with the own window complete.  A
+  // wait that ran out is reported at the next common decision.
+  auto publish = [&] {
+#pragma unroll
+    for (int u = 0; u < kClOwn; ++u)
+      if (tid + u * T < R) pw_s[own + tid + u * T] = p[u];
+    if (tid == 0) cl_expect(bar_p, (uint32_t)(wn - R) * (uint32_t)sizeof(double));
+    __syncthreads();
+    for (int c = warp; c < (int)NC; c += W) {
+      if (c == (int)rank) continue;
+      const int c0 = all_s[c][0], hi = min((int)row_lo + R, all_s[c][1]);
+      for (int i = max((int)row_lo, c0) + lane; i < hi; i += 32)
+        cl_send(pw_base + (uint32_t)(i - c0) * 8u, bar_p, c, pw_s[i - w0]);
+    }
+    if (!cl_wait(bar_p, phase_p)) fail_s = 1;
+    phase_p ^= 1;
+  };
+#pragma unroll
+  for (int u = 0; u < kClOwn; ++u) {
+    const int a = tid + u * T;
+    x[u] = r[u] = mi[u] = 0.0;
+    if (a < R) {
+      r[u] = P.b[row_lo + a];
+      mi[u] = P.dinv[row_lo + a];
+    }
+    p[u] = z[u] = mi[u] * r[u];
+  }
+  publish();
+  // r.z and r.r over all rows: every warp sends its shares to every CTA, where
+  // warp 0 sums r.z and warp 1 r.r.  pre() runs while the words travel.
+  uint32_t phase_b = 0;
+  double total = 0.0;  // warp 0: r.z, warp 1: r.r
+  auto reduce_rz_rr = [&](auto&& pre) {
+    if (tid == 0) cl_expect(bar_b, 2 * n_b * (uint32_t)sizeof(double));
+    if (nu > 0) {
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < kClOwn; ++u) {
+        if (u >= nu) break;
+        s.x = u ? fma(r[u], z[u], s.x) : r[u] * z[u];
+        s.y = u ? fma(r[u], r[u], s.y) : r[u] * r[u];
+      }
+      s = warp_sum_fixed2(s.x, s.y);
+      if ((lane & 15) < (int)NC)
+        cl_send(smem_u32(&part[1 + (lane >> 4)][at_b + warp]), bar_b, lane & 15, lane < 16 ? s.x : s.y);
+    }
+    pre();
+    if (warp < 2) {
+      if (!cl_wait(bar_b, phase_b)) fail_s = 1;
+      total = cl_total(part[1 + warp], n_b);
+    }
+    phase_b ^= 1;
+  };
+  reduce_rz_rr([] {});
+  double rz = total;              // of warp 0
+  double bb = total, tol2 = 0.0;  // of warp 1
+  long long iters = 0;
+  if (tid == 0) {
+    sh_done[0] = fail_s ? kDoneBarrierTimeout : finite_bits(rz) ? kDoneNo : kDoneNonFinite;
+    sh_rz = rz;
+  }
+  if (tid == 32) {
+    tol2 = P.rtol2 * bb;
+    sh_done[1] = !finite_bits(bb) ? kDoneNonFinite : (bb == 0.0 || bb <= tol2) ? kDoneConverged : kDoneNo;
+  }
+  __syncthreads();
+  int done = sh_done[0] ? sh_done[0] : sh_done[1];
+  uint32_t phase_a = 0;
+  while (done == kDoneNo) {
+    // ---- q = A p on L lanes per row, this warp's share of p.q
+    double pq = 0.0;
+    if (tid == 0) cl_expect(bar_a, n_a * (uint32_t)sizeof(double));
+    for (int k = warp; k < nb; k += W) {
+      const int b0 = base_s[k], steps = base_s[k + 1] - b0;
+      const double* v = val_s + (size_t)b0 * 32 + lane;
+      const uint16_t* c = code_s + (size_t)b0 * 32 + lane;
+      double s = 0.0;
+#pragma unroll 8
+      for (int j = 0; j < steps; ++j) s = fma(v[j * 32], pw_s[c[j * 32]], s);
+      for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, L);
+      const int slot = k * rpb + (lane >> lsh);
+      if ((lane & (L - 1)) == 0 && slot < R) {
+        const int row = row_s[slot];
+        q_s[row] = s;
+        pq = fma(pw_s[own + row], s, pq);
+      }
+    }
+    if (warp < nb) {
+      pq = warp_sum_fixed(pq);
+      if (lane < (int)NC) cl_send(smem_u32(&part[0][at_a + warp]), bar_a, lane, pq);
+    }
+    if (warp == 0) {
+      if (!cl_wait(bar_a, phase_a)) fail_s = 1;
+      const double v = cl_total(part[0], n_a);
+      if (lane == 0) {
+        sh_scalar = rz / v;  // alpha
+        sh_done[0] = fail_s ? kDoneBarrierTimeout : !finite_bits(v) ? kDoneNonFinite : zero_bits(v) ? kDoneBreakdown
+                                                                                                    : kDoneNo;
+      }
+    } else if (tid == T - 1) {
+      sh_inv = 1.0 / sh_rz;
+    }
+    phase_a ^= 1;
+    __syncthreads();
+    done = sh_done[0];
+    if (done != kDoneNo) break;
+    // ---- x += alpha p, r -= alpha q, z = M r
+    const double alpha = sh_scalar;
+#pragma unroll
+    for (int u = 0; u < kClOwn; ++u) {
+      if (u >= nu) break;
+      const int a = tid + u * T;
+      r[u] = fma(-alpha, a < R ? q_s[a] : 0.0, r[u]);
+      z[u] = mi[u] * r[u];
+    }
+    reduce_rz_rr([&] {
+#pragma unroll
+      for (int u = 0; u < kClOwn; ++u) {
+        if (u >= nu) break;
+        x[u] = fma(alpha, p[u], x[u]);
+      }
+    });
+    iters += 1;
+    if (tid == 0) {
+      sh_done[0] = fail_s ? kDoneBarrierTimeout : finite_bits(total) ? kDoneNo : kDoneNonFinite;
+      sh_scalar = total * sh_inv;  // beta
+      sh_rz = rz = total;
+    }
+    if (tid == 32)
+      sh_done[1] = !finite_bits(total) ? kDoneNonFinite
+                   : total <= tol2 ? kDoneConverged
+                   : iters >= P.max_iter ? kDoneMaxIter : kDoneNo;
+    __syncthreads();
+    done = sh_done[0] ? sh_done[0] : sh_done[1];
+    if (done != kDoneNo) break;
+    const double beta = sh_scalar;
+#pragma unroll
+    for (int u = 0; u < kClOwn; ++u) {
+      if (u >= nu) break;
+      p[u] = fma(beta, p[u], z[u]);
+    }
+    publish();
+  }
+#pragma unroll
+  for (int u = 0; u < kClOwn; ++u)
+    if (tid + u * T < R) P.x[row_lo + tid + u * T] = x[u];
+  if (rank == 0 && tid == 32) {
+    P.ctrl->iters = iters;
+    P.ctrl->rr = total;
+    P.ctrl->bb = bb;
+    P.ctrl->rscale = 1.0;
+    P.ctrl->done = done;
+  }
+  cl_sync();  // no CTA leaves while another may still send to it
+}
+
 // ------------------------------------------------------------------ MINRES --
 // Jacobi-preconditioned MINRES (Paige & Saunders, SIAM J. Numer. Anal. 12,
 // 1975) on the FP64 CSR matrix: the reference's GPU `method="minres"`
@@ -1891,6 +2362,74 @@ static int iterate(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT* q, doubl
   return FEM_OK;
 }
 
+// CTAs per cluster that the device can place for the one-cluster CG (16, else
+// 8, else none), looked up once per host thread.
+static int cluster_size() {
+  static thread_local int size = -1;
+  if (size < 0) {
+    size = 0;
+    if (cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kClSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+      for (int c = kClMax; c >= 8 && size == 0; c /= 2) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = c;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(kClThreads);
+        cfg.dynamicSmemBytes = kClSmem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_pcg_cluster, &cfg) == cudaSuccess && n >= 1) size = c;
+      }
+    }
+    cudaGetLastError();
+  }
+  return size;
+}
+
+// One-cluster solve of a small CSR system; *ran false leaves the system to
+// the grid-wide path (too many rows, or declined on the device).
+static int cluster_pcg(const fem_matrix* A, const double* b, double* x, double rtol, int64_t max_iter, Ctrl* ctrl,
+                       Ctrl* h, bool timing, bool* ran, cudaStream_t st) {
+  *ran = false;
+  if (!use_persistent() || A->n > (int64_t)kClMax * kClRows) return FEM_OK;
+  const ClusterParams P = {A->n, A->row_ptr, A->col, (const double*)A->val, (const double*)A->precond, b, x, ctrl,
+                           rtol * rtol, (long long)max_iter};
+  const int c = cluster_size();
+  if (c == 0) return FEM_OK;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = c;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(c);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = kClSmem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (timing) cudaEventRecord(g_timer.ev[0], st);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_pcg_cluster, P);
+  ::tfg::note_launch();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return FEM_OK;
+  }
+  if (timing) cudaEventRecord(g_timer.ev[1], st);
+  const int rd = read_ctrl(ctrl, h, st);
+  if (rd) return rd;
+  *ran = h->done != kClNoFit;
+  float t = 0.f;
+  if (timing && *ran && cudaEventElapsedTime(&t, g_timer.ev[0], g_timer.ev[1]) == cudaSuccess) {
+    g_timer.ms += t;
+    g_timer.timed += h->iters;
+  }
+  return FEM_OK;
+}
+
 struct Vecs {
   Ctrl* ctrl;
   void *x, *r, *z, *p, *q;
@@ -1930,34 +2469,43 @@ static int run_pcg(const fem_matrix* A, const double* b, double* x, double rtol,
                    const Vecs& v, fem_solve_info* info, cudaStream_t st, bool timing_on) {
   Ctrl h;
   memset(&h, 0, sizeof(h));
-  h.max_iter = max_iter;
-  h.mixed = 0;
-  h.rscale = 1.0;
-  if (cudaMemcpyAsync(v.ctrl, &h, sizeof(Ctrl), cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return check_cuda("fem_pcg ctrl");
-  VT* xv = (G == 1) ? reinterpret_cast<VT*>(x) : reinterpret_cast<VT*>(v.x);
-  const int64_t ng = A->n / G;
-  g_persistent_refused = false;
-  if (sizeof(VT) == 4) {  // FP32 vectors iterate on b scaled to near unit norm
-    k_bnorm<<<vec_grid(A->n), kThreads, 0, st>>>(A->n, b, v.partial, v.ctrl);
-    ::tfg::note_launch();
-  }
-  k_init<G, VT><<<grid_for(ng, kThreads), kThreads, 0, st>>>(
-      ng, b, xv, (VT*)v.r, (VT*)v.z, (VT*)v.p, A->precond, v.partial, v.ctrl, rtol * rtol);
-      ::tfg::note_launch();
-  TFG_CHECK_LAUNCH("fem_pcg init");
-  int rc = read_ctrl(v.ctrl, &h, st);
-  if (rc) return rc;
   const bool timing = timing_on && g_timer.init() == FEM_OK;
   if (timing) {
     g_timer.ms = 0.0;
     g_timer.timed = 0;
   }
-  int chunk = 8;
-  while (h.done == kDoneNo) {
-    rc = iterate<G, VT>(A, xv, (VT*)v.r, (VT*)v.z, (VT*)v.p, (VT*)v.q, v.partial, v.ctrl, &h, timing,
-                        &chunk, st);
+  int rc;
+  bool solved = false;
+  if constexpr (G == 1) {
+    rc = cluster_pcg(A, b, x, rtol, max_iter, v.ctrl, &h, timing, &solved, st);
     if (rc) return rc;
+  }
+  if (!solved) {
+    memset(&h, 0, sizeof(h));
+    h.max_iter = max_iter;
+    h.mixed = 0;
+    h.rscale = 1.0;
+    if (cudaMemcpyAsync(v.ctrl, &h, sizeof(Ctrl), cudaMemcpyHostToDevice, st) != cudaSuccess)
+      return check_cuda("fem_pcg ctrl");
+    VT* xv = (G == 1) ? reinterpret_cast<VT*>(x) : reinterpret_cast<VT*>(v.x);
+    const int64_t ng = A->n / G;
+    g_persistent_refused = false;
+    if (sizeof(VT) == 4) {  // FP32 vectors iterate on b scaled to near unit norm
+      k_bnorm<<<vec_grid(A->n), kThreads, 0, st>>>(A->n, b, v.partial, v.ctrl);
+      ::tfg::note_launch();
+    }
+    k_init<G, VT><<<grid_for(ng, kThreads), kThreads, 0, st>>>(
+        ng, b, xv, (VT*)v.r, (VT*)v.z, (VT*)v.p, A->precond, v.partial, v.ctrl, rtol * rtol);
+    ::tfg::note_launch();
+    TFG_CHECK_LAUNCH("fem_pcg init");
+    rc = read_ctrl(v.ctrl, &h, st);
+    if (rc) return rc;
+    int chunk = 8;
+    while (h.done == kDoneNo) {
+      rc = iterate<G, VT>(A, xv, (VT*)v.r, (VT*)v.z, (VT*)v.p, (VT*)v.q, v.partial, v.ctrl, &h, timing,
+                          &chunk, st);
+      if (rc) return rc;
+    }
   }
   if (G != 1) k_copy_cast<<<grid_for(A->n, kThreads), kThreads, 0, st>>>(A->n, (const float*)v.x, x, v.ctrl);
   ::tfg::note_launch();
