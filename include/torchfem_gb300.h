@@ -80,7 +80,7 @@ enum {
 };
 
 enum { FEM_F64 = 0, FEM_F32 = 1 };
-enum { FEM_FMT_CSR_F64 = 1, FEM_FMT_SELL_F32 = 2 };
+enum { FEM_FMT_CSR_F64 = 1, FEM_FMT_SELL_F32 = 2, FEM_FMT_SELL_F64 = 3 };
 
 /* Last error message of the calling thread (host string). */
 const char* fem_last_error(void);
@@ -399,14 +399,14 @@ int fem_block_jacobi(const fem_blocks* blocks, const float* sval, const int64_t*
 /* ------------------------------------------------------------------------ */
 
 typedef struct fem_matrix {
-  int format;              /* FEM_FMT_CSR_F64 or FEM_FMT_SELL_F32 */
-  int block;               /* 1 for CSR, dim for the sliced block layout */
+  int format;              /* FEM_FMT_CSR_F64, FEM_FMT_SELL_F32 or FEM_FMT_SELL_F64 */
+  int block;               /* 1 for CSR, DOFs per node for the sliced block layouts */
   int64_t n;               /* unknowns */
   int64_t n_rows;          /* scalar rows (CSR) or node rows (sliced) */
   const int64_t* row_ptr;  /* CSR row pointers [n_rows+1] or sell_base [n_slices+1] */
   const int32_t* col;      /* scalar column ids or slot columns */
-  const void* val;         /* FP64 [nnz] or FP32 sliced block values */
-  const void* precond;     /* FP64 inverse diagonal [n] or FP32 inverse blocks */
+  const void* val;         /* FP64 [nnz] or FP32 / FP64 sliced block values */
+  const void* precond;     /* FP64 inverse diagonal [n] (FP64 formats) or FP32 inverse blocks */
 } fem_matrix;
 
 typedef struct fem_solve_info {
@@ -497,6 +497,13 @@ typedef struct fem_operator64 {
 size_t fem_apply64_workspace_bytes(const fem_operator64* op);
 int fem_apply64(const fem_operator64* op, const double* x, double* y, void* ws, size_t ws_bytes,
                 void* stream);
+
+/* FP64 CSR values (fem_assemble_csr's order) into the sliced block layout,
+ * sval64 [n_slots * dim^2], padding zero: the FEM_FMT_SELL_F64 form of the
+ * same matrix, with which fem_pcg runs faster on systems beyond the reach of
+ * its one-cluster kernel.  dim 1..3. */
+int fem_csr_to_sell64(const fem_blocks* blocks, const int64_t* row_ptr, const double* val,
+                      const int64_t* sell_base, double* sval64, void* stream);
 
 /* y = A x in FP64 over the FP64 copy of a sliced matrix
  * (fem_assemble_sell_pair), with the layout of the FP32 sliced

@@ -255,8 +255,7 @@ struct Ctrl {
   int replace;
   int mixed;
   unsigned int counter;
-  int bar_error;             // persistent kernel: a barrier wait ran out
-  unsigned long long bar_seq;  // persistent kernel: grid-barrier arrivals, never reset within a solve
+  int bar_error;             // persistent kernel: a grid-wide wait ran out
 };
 
 // Two block sums in one pass (fixed order).  Valid in thread 0.
@@ -692,8 +691,8 @@ __global__ void k_copy_cast(int64_t n, const float* __restrict__ in, double* __r
 // replacement (mixed) or the iteration cap.  Each CTA owns a contiguous range
 // of rows (slices for the sliced layout): it computes q = A p for them, then
 // updates x, r, z and p for the same rows, so the only data crossing CTAs are
-// the gathered p values and three scalars per iteration.  Three grid barriers
-// per iteration; every CTA sums the per-CTA partials itself in one fixed
+// the gathered p values and three scalars per iteration.  Two grid sums and a barrier
+// per iteration; every CTA sums the per-CTA shares itself in one fixed
 // order, so all CTAs take identical decisions and results are deterministic.
 // The matrix is streamed with L2 evict_first; the CG vectors stay in L2.
 constexpr int kCsrTpr = 8;  // lanes per scalar CSR row
@@ -723,88 +722,245 @@ struct PersistParams {
   void* z;
   void* p;
   void* q;
-  double* partial;  // [3 * gridDim.x]
+  unsigned long long* sync;  // of GridSync, zeroed before the launch
   Ctrl* ctrl;
-  long long spin_limit;  // clock cycles a barrier wait may last
+  long long spin_limit;  // clock cycles a grid-wide wait may last
 };
 
-// Grid barrier with a bounded wait, fused with the fixed-order sum of NK
-// per-CTA partials.  One monotonic 64-bit arrival counter: every CTA adds 1
-// (release) and polls (relaxed, with a short sleep, so that polling neither
-// floods the counter's L2 slice nor invalidates L1 lines a co-resident CTA is
-// using) until the count reaches the next multiple of the grid size; one
-// acquire fence follows.  No reset step sits on the critical path: the counter
-// starts at 0 for each solve and every launch passes whole barriers only.
-// Then warp 0 alone sums partial[3*i + k0 + j] over the CTAs i in one fixed
-// order and shares the sums through shared memory, so every thread of every
-// CTA holds identical values.  Returns false (on every thread) once any CTA's
-// wait has run out; the kernel then stops.
-template <int NK, typename F>
-__device__ __forceinline__ bool grid_barrier(Ctrl* c, long long spin_limit, const double* partial, int k0, F&& on_sums) {
+// Sums of K doubles per lane on the integer pipe, the same values in every
+// lane: each is aligned to its largest exponent as a 58-bit integer (five
+// bits below an FP64 mantissa, rounded to nearest), added exactly in three
+// redux words and rounded to FP64 once.  The error is at most 32 half units
+// of 2^-58 of the largest value plus that rounding, no more than five FP64
+// additions leave.  Exponents at either end of the range (and NaN,
+// infinities) take the FP64 tree.
+template <int K>
+__device__ __forceinline__ void sum_fixed(double (&v)[K]) {
+  int ex[K], e[K];
+  bool plain = true;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    ex[k] = (__double2hiint(v[k]) >> 20) & 0x7ff;
+    e[k] = (int)__reduce_max_sync(0xffffffffu, (unsigned)ex[k]);
+    plain = plain && e[k] >= 128 && e[k] <= 1990;
+  }
+  if (!plain) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      v[k] = __any_sync(0xffffffffu, (__double_as_longlong(v[k]) << 1) != 0) ? warp_sum(v[k]) : 0.0;
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const long long bits = __double_as_longlong(v[k]);
+    const int sh = min(e[k] - ex[k], 62);
+    unsigned long long m = ((unsigned long long)(bits & 0xfffffffffffffLL) | (1ull << 52)) << 5;
+    m = ex[k] == 0 ? 0ull : (m + ((1ull << sh) >> 1)) >> sh;
+    const long long f = bits < 0 ? -(long long)m : (long long)m;
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)f & 0x3fffffu);
+    const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 22) & 0x3fffffu);
+    const int hi = __reduce_add_sync(0xffffffffu, (int)(f >> 44));
+    const long long t = ((long long)hi << 44) + ((long long)mid << 22) + (long long)lo;
+    v[k] = t == 0 ? 0.0 : __longlong_as_double(__double_as_longlong((double)t) + ((long long)(e[k] - 1080) << 52));
+  }
+}
+
+// Kept out of line: an iteration calls them several times, and straight-line code
+// that runs once an iteration is fetched more slowly than it executes.
+__device__ __noinline__ double warp_sum_fixed(double a) {
+  double v[1] = {a};
+  sum_fixed<1>(v);
+  return v[0];
+}
+__device__ __noinline__ double2 warp_sum_fixed2(double a, double b) {
+  double v[2] = {a, b};
+  sum_fixed<2>(v);
+  return make_double2(v[0], v[1]);
+}
+
+// isfinite and == 0 by the bits: a comparison costs an FP64 instruction.
+__device__ __forceinline__ bool finite_bits(double v) { return ((__double2hiint(v) >> 20) & 0x7ff) != 0x7ff; }
+__device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
+
+// Grid-wide sums and barriers of the persistent kernels, with bounded waits.
+//
+// grid_barrier: one counter, a release reduction and acquire polls (2,500
+// cycles on 152 CTAs); it orders the CTA's writes before the other CTAs'
+// reads after it.
+//
+// grid_sum: the sum of NK doubles per CTA in one hop, by the counter itself.
+// Each value is added as a 144-bit fixed-point number in four words, 36 bits to
+// a word above an 18-bit count of arrivals, so the word that a CTA polls for the
+// last arrival already holds the sum: no release, no second trip for the
+// values, no additions by the reader (1,700 cycles for the hop; 4,500 with
+// per-CTA partials behind a counter; polling every CTA's own slot, 3,400,
+// since 152 pollers queue at the slots' L2 lines).  Integer additions commute:
+// the sum does not depend on the order of arrival.  The fixed point's scale
+// comes from the last sum of the same quantity, known to all: 2^-97 of it is
+// the unit, and a share up to 2^40 times as large fits.  A share beyond that
+// or not finite is marked in the words (nine bits above the count), and then,
+// like a first sum without a scale, the doubles themselves go round
+// (grid_sum_plain).  The words only ever grow and are read as differences; two
+// sets alternate, since a CTA that adds to one again has seen every CTA in the
+// other, hence every CTA has read the first.
+constexpr int kSumWords = 4, kSumBits = 36;
+constexpr int kSumLine = 16;                                   // 8-byte words from one to the next
+constexpr int kSumHead = kSumLine * (1 + 2 * 2 * kSumWords);   // the counter, 2 sets of 2 values; plain slots follow
+struct GridSync {
+  unsigned long long* mem;      // zeroed before the launch
+  unsigned long long prev0, prev1;  // warp 0: this lane's word of either set at its last sum
+  unsigned long long barriers;  // barriers passed (thread 0)
+  uint32_t sums, plain;         // sums so far, those of them by plain doubles
+};
+__device__ __forceinline__ void grid_sync_init(GridSync& g, unsigned long long* mem) {
+  g.mem = mem;
+  g.prev0 = g.prev1 = g.barriers = 0;
+  g.sums = g.plain = 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(Ctrl* c, long long spin_limit, GridSync& g) {
   __shared__ int ok;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    if (threadIdx.x == 0) {
-      unsigned long long old;
-      asm volatile("atom.add.release.gpu.u64 %0, [%1], 1;" : "=l"(old) : "l"(&c->bar_seq) : "memory");
-      const unsigned long long target = (old / gridDim.x + 1) * gridDim.x;
-      const long long t0 = clock64();
-      while (true) {
-        unsigned long long now;
-        asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(now) : "l"(&c->bar_seq) : "memory");
-        if (now >= target) break;
-        if (*(volatile int*)&c->bar_error) break;
-        if (clock64() - t0 > spin_limit) {
-          atomicExch(&c->bar_error, 1);
-          break;
-        }
-        __nanosleep(32);
+  if (threadIdx.x == 0) {
+    g.barriers += gridDim.x;
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(g.mem) : "memory");
+    const long long t0 = clock64();
+    bool good = true;
+    while (true) {
+      unsigned long long now;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(g.mem) : "memory");
+      if (now >= g.barriers) break;
+      if (clock64() - t0 > spin_limit) {
+        good = false;
+        break;
       }
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      ok = (*(volatile int*)&c->bar_error) == 0;
     }
-    __syncwarp();
-    if constexpr (NK > 0) {
-      const int lane = threadIdx.x;
-      double sums[NK];
-#pragma unroll
-      for (int j = 0; j < NK; ++j) {
-        double v = 0.0;
-        for (int i = lane; i < (int)gridDim.x; i += 32) v += __ldcg(partial + 3 * i + k0 + j);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        sums[j] = v;
-      }
-      if (lane == 0) on_sums(sums);
-    }
+    if (!good) atomicExch(&c->bar_error, 1);
+    ok = good;
   }
   __syncthreads();
   return ok != 0;
 }
 
-// Fixed-order CTA sum of N per-thread accumulators: shuffle tree within each
-// warp, then thread 0 adds the warp sums in FP64 and stores them to out[j].
-template <int N, typename ACC>
-__device__ __forceinline__ void cta_partials(ACC (&v)[N], double* out, double (*wsum)[2]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[j].shfl_down(o);
+// The sum of the doubles themselves, each to its CTA's slot as two words of half
+// a value and a sequence number; warp 0 of every CTA.
+struct PlainSum {
+  double x, y;
+  int good;
+};
+template <int NK>
+__device__ __noinline__ PlainSum grid_sum_plain(unsigned long long* mem, uint32_t seq, long long spin_limit, double x,
+                                                double y) {
+  const int lane = threadIdx.x & 31, NC = gridDim.x;
+  ulonglong2* buf = reinterpret_cast<ulonglong2*>(mem + kSumHead) + (size_t)(seq & 1) * NC * 2;
+  if (lane < NK) {
+    const unsigned long long w = (unsigned long long)__double_as_longlong(lane ? y : x);
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(buf + (size_t)blockIdx.x * 2 + lane),
+                 "l"((w << 32) | seq), "l"((w & 0xffffffff00000000ull) | seq)
+                 : "memory");
   }
-  if (lane == 0) {
+  bool good = true;
+  double sums[NK];
+  const long long t0 = clock64();
 #pragma unroll
-    for (int j = 0; j < N; ++j) wsum[warp][j] = v[j].value();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w][j];
-      out[j] = t;
+  for (int j = 0; j < NK; ++j) {
+    sums[j] = 0.0;
+    for (int i = lane; i < NC; i += 32) {
+      unsigned long long a, b;
+      while (true) {
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                     : "=l"(a), "=l"(b)
+                     : "l"(buf + (size_t)i * 2 + j)
+                     : "memory");
+        if ((uint32_t)a == seq && (uint32_t)b == seq) break;
+        if (clock64() - t0 > spin_limit) {
+          good = false;
+          break;
+        }
+      }
+      sums[j] += __longlong_as_double((long long)((a >> 32) | (b & 0xffffffff00000000ull)));
     }
   }
+  PlainSum t;
+  t.good = __all_sync(0xffffffffu, good);
+  t.x = warp_sum_fixed(sums[0]);
+  t.y = NK > 1 ? warp_sum_fixed(sums[NK - 1]) : 0.0;
+  return t;
+}
+
+// mine: this CTA's values, on every lane of warp 0.  ref: the scale of this
+// quantity (of lane j: of value j / 4), 0 at first.  on_sums runs in thread 0,
+// with the same sums on every CTA.  False (on every thread) if the wait ran
+// out; the kernel then stops, and so, by their own limits, do the other CTAs.
+template <int NK, typename F>
+__device__ __forceinline__ bool grid_sum(Ctrl* c, long long spin_limit, GridSync& g, const double (&mine)[NK],
+                                         int& ref, F&& on_sums) {
+  __shared__ int ok;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, word = lane & (kSumWords - 1);
+    const bool part = lane < NK * kSumWords;
+    const uint32_t set = ++g.sums & 1;
+    bool good = true, plain = __any_sync(0xffffffffu, part && ref == 0);
+    double v[NK];
+#pragma unroll
+    for (int j = 0; j < NK; ++j) v[j] = mine[j];
+    if (!plain) {
+      unsigned long long delta = 0;
+      if (part) {
+        const long long bits = __double_as_longlong(lane < kSumWords ? mine[0] : mine[NK - 1]);
+        const int ex = (int)((bits >> 52) & 0x7ff);
+        const unsigned long long m = ex == 0 ? 0ull : (unsigned long long)(bits & 0xfffffffffffffLL) | (1ull << 52);
+        const bool off = ex - ref > 40;  // includes the exponent of infinities and NaN
+        const int sh = ex - ref + 45 - kSumBits * word;
+        unsigned long long q = off || sh <= -53 || sh >= kSumBits ? 0ull : sh < 0 ? m >> -sh : m << sh;
+        q &= (1ull << kSumBits) - 1;
+        if (bits < 0) q = 0ull - q;
+        unsigned long long* at = g.mem + kSumLine * (1 + (int)set * 2 * kSumWords + lane);
+        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(at), "l"((q << 18) + (off ? 513ull : 1ull))
+                     : "memory");
+        const long long t0 = clock64();
+        const unsigned long long before = set ? g.prev1 : g.prev0;
+        unsigned long long now;
+        while (true) {
+          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(at) : "memory");
+          delta = now - before;
+          if ((delta & 511) == gridDim.x) break;
+          if (clock64() - t0 > spin_limit) {
+            good = false;
+            break;
+          }
+        }
+        if (set) g.prev1 = now;
+        else g.prev0 = now;
+      }
+      __syncwarp();
+      good = __all_sync(0xffffffffu, good);
+      plain = __any_sync(0xffffffffu, ((delta >> 9) & 511) != 0);
+      const long long sum = (long long)delta >> 18;
+      double d = sum == 0 ? 0.0
+                          : __longlong_as_double(__double_as_longlong((double)sum) +
+                                                 ((long long)(kSumBits * word + ref - 1120) << 52));
+      d += __shfl_xor_sync(0xffffffffu, d, 1);
+      d += __shfl_xor_sync(0xffffffffu, d, 2);
+#pragma unroll
+      for (int j = 0; j < NK; ++j) v[j] = __shfl_sync(0xffffffffu, d, j * kSumWords);
+    }
+    if (plain && good) {
+      const PlainSum t = grid_sum_plain<NK>(g.mem, ++g.plain, spin_limit, mine[0], mine[NK - 1]);
+      v[0] = t.x;
+      if constexpr (NK > 1) v[1] = t.y;
+      good = t.good;
+    }
+    const int e = (__double2hiint(lane < kSumWords ? v[0] : v[NK - 1]) >> 20) & 0x7ff;
+    ref = e >= 256 && e <= 1900 ? e : 0;
+    if (lane == 0) {
+      if (!good) atomicExch(&c->bar_error, 1);
+      ok = good;
+      on_sums(v);
+    }
+  }
+  __syncthreads();
+  return ok != 0;
 }
 
 // Dot-product accumulators of the persistent CG.  On the FP32 (mixed) path a
@@ -815,6 +971,7 @@ __device__ __forceinline__ void cta_partials(ACC (&v)[N], double* out, double (*
 // plain double.
 template <typename VT> struct DotAcc;
 template <> struct DotAcc<double> {
+  static constexpr bool kPlain = true;
   double v = 0.0;
   __device__ __forceinline__ void fma(double a, double b) { v = ::fma(a, b, v); }
   __device__ __forceinline__ void shfl_down(int o) { v += __shfl_down_sync(0xffffffffu, v, o); }
@@ -827,6 +984,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 template <> struct DotAcc<float> {
+  static constexpr bool kPlain = false;
   float hi = 0.f, lo = 0.f;
   __device__ __forceinline__ void add(float x, float x_lo) {
     float s, e;
@@ -848,6 +1006,46 @@ template <> struct DotAcc<float> {
   }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
+
+// Fixed-order CTA sum of N per-thread accumulators (N = 1 or 2): within each
+// warp, then over the warp sums on warp 0, whose lanes hold the result.
+template <int N, typename ACC>
+__device__ __forceinline__ void cta_partials(ACC (&v)[N], double (&out)[N], double (*wsum)[2]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(N == 1 || N == 2, "one or two sums");
+  double s[2] = {0.0, 0.0};
+  if constexpr (ACC::kPlain) {
+    if constexpr (N == 2) {
+      const double2 t = warp_sum_fixed2(v[0].value(), v[1].value());
+      s[0] = t.x;
+      s[1] = t.y;
+    } else {
+      s[0] = warp_sum_fixed(v[0].value());
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[j].shfl_down(o);
+      s[j] = v[j].value();
+    }
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) wsum[warp][j] = s[j];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int nw = blockDim.x >> 5;
+    if constexpr (N == 2) {
+      const double2 t = warp_sum_fixed2(lane < nw ? wsum[lane][0] : 0.0, lane < nw ? wsum[lane][1] : 0.0);
+      out[0] = t.x;
+      out[1] = t.y;
+    } else {
+      out[0] = warp_sum_fixed(lane < nw ? wsum[lane][0] : 0.0);
+    }
+  }
+}
 
 // First i in [0, n] with base[i] >= target (base non-decreasing).
 __device__ __forceinline__ int64_t lower_bound_i64(const int64_t* base, int64_t n, int64_t target) {
@@ -1172,6 +1370,9 @@ __global__ void __launch_bounds__(kPThreads, MODE == 1 ? 1 : 2) k_pcg_persistent
   // drift measurably degrades tight tolerances, so it keeps three barriers.
   constexpr bool kCarry = MODE == 1 && G == 3 && sizeof(VT) == 4;
   bool carry = false;
+  GridSync sync;
+  grid_sync_init(sync, P.sync);
+  int ref1 = 0, ref2 = 0;
   if (threadIdx.x == 0) sh_beta = (VT)0;
   __syncthreads();
   while (true) {
@@ -1354,8 +1555,9 @@ __global__ void __launch_bounds__(kPThreads, MODE == 1 ? 1 : 2) k_pcg_persistent
         __syncthreads();
       }
     }
-    cta_partials<1, ACC>(pq, P.partial + 3 * cta, wsum);
-    const bool ok1 = grid_barrier<1>(c, P.spin_limit, P.partial, 0, [&](const double* sm) {
+    double share1[1];
+    cta_partials<1, ACC>(pq, share1, wsum);
+    const bool ok1 = grid_sum<1>(c, P.spin_limit, sync, share1, ref1, [&](const double* sm) {
       const double pq_tot = sm[0];
       if (pq_tot == 0.0 || !isfinite(pq_tot)) {
         sh_stop = 1;
@@ -1380,8 +1582,9 @@ __global__ void __launch_bounds__(kPThreads, MODE == 1 ? 1 : 2) k_pcg_persistent
       for (int64_t a = row_lo + threadIdx.x; a < row_hi; a += blockDim.x)
         node_update<G, VT>(P.prec, a, alpha, x, r, z, p, q, rzrr[0], rzrr[1]);
     }
-    cta_partials<2, ACC>(rzrr, P.partial + 3 * cta + 1, wsum);
-    const bool ok2 = grid_barrier<2>(c, P.spin_limit, P.partial, 1, [&](const double* sm) {
+    double share2[2];
+    cta_partials<2, ACC>(rzrr, share2, wsum);
+    const bool ok2 = grid_sum<2>(c, P.spin_limit, sync, share2, ref2, [&](const double* sm) {
       const double rz_new = sm[0], rr = sm[1];
       iters += 1;
       int stop = 0;  // 1 done, 2 replace
@@ -1424,12 +1627,12 @@ __global__ void __launch_bounds__(kPThreads, MODE == 1 ? 1 : 2) k_pcg_persistent
     });
     if (!ok2 || sh_stop) break;
     if constexpr (kCarry) {
-      carry = true;  // the next SpMV applies p = z + beta p itself
+      carry = true;  // the next SpMV gathers z and applies p = z + beta p itself
     } else {
       // ---- phase C: p = z + beta p on own rows
       direction_update<VT, MODE == 1 ? 4 : 2>(p, z, sh_beta, row_lo * G, row_hi * G);
-      if (!grid_barrier<0>(c, P.spin_limit, nullptr, 0, [](const double*) {})) break;
     }
+    if (!grid_barrier(c, P.spin_limit, sync)) break;
   }
   if constexpr (MODE == 1) {
     // wait for this warp's prefetched chunks before the CTA exits
@@ -1439,6 +1642,224 @@ __global__ void __launch_bounds__(kPThreads, MODE == 1 ? 1 : 2) k_pcg_persistent
     }
   }
   if (cta == 0 && threadIdx.x == 0 && *(volatile int*)&c->bar_error) c->done = kDoneBarrierTimeout;
+}
+
+// ------------------------------------------------ FP64 sliced-block CG ------
+// The plain FP64 CG on the sliced block layout (fem_csr_to_sell64), for
+// systems of node blocks beyond the one-cluster kernel.  Same shape as
+// k_pcg_persistent; what differs is the product.  The FP64 unit (two lanes a
+// clock) bounds it: the CSR form spends it on the lane sums of its eight lanes
+// per row and on half-empty last passes (about half of its FP64 instructions),
+// a thread per row on nothing but the stored values, and a node's columns are
+// loaded and its p gathered once per block.  KS warps share a slice: four, one
+// per sub-partition of the SM, so that a CTA's few slices load the four FP64
+// units evenly (their partial rows meet in shared memory), or one where there
+// are slices enough (launch_sell64).  x lags one direction: x += alpha p is
+// applied where p is read anyway.  Per iteration, CSR kernel before and this:
+// 51.5 -> 30 us at 118k unknowns (33^3), 127 -> 79 us at 447k (52^3), 282 ->
+// 180 us at 1.07M (70^3; 95 M FP64 FMA, 151 us at two lanes a clock).
+template <int D, int KS>
+__global__ void __launch_bounds__(kPThreads, 1) k_pcg_sell64(PersistParams P) {
+  constexpr int DD = D * D, NW = kPThreads / 32, NG = NW / KS;
+  __shared__ double wsum[NW][2];
+  __shared__ double ys[KS > 1 ? 2 : 1][KS > 1 ? NW : 1][D][32];
+  __shared__ double sh_alpha, sh_beta, sh_rz, sh_inv;
+  __shared__ int sh_stop;
+  Ctrl* c = P.ctrl;
+  if (ctrl_idle(c)) return;
+  const int cta = blockIdx.x, NC = gridDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = warp / KS, kofs = warp % KS;
+  double* __restrict__ x = (double*)P.x;
+  double* __restrict__ r = (double*)P.r;
+  double* __restrict__ z = (double*)P.z;
+  double* __restrict__ p = (double*)P.p;
+  double* __restrict__ q = (double*)P.q;
+  const double* __restrict__ dinv = (const double*)P.prec;
+  const double* __restrict__ val = (const double*)P.val;
+  const uint64_t stream = l2_policy(false);
+  const int64_t ns = (P.n_rows + 31) >> 5;
+  // slices of this CTA: equal shares of the slot-rows plus a slice's fixed cost
+  // of about three (its sums, p.q and the loads' latency): slices at the mesh
+  // boundary are short
+  constexpr int64_t kFixed = 3 * 32;
+  const int64_t work = P.row_ptr[ns] + kFixed * ns;
+  auto bound = [&](int64_t target) {
+    int64_t a = 0, b = ns;
+    while (a < b) {
+      const int64_t mid = (a + b) >> 1;
+      if (P.row_ptr[mid] + kFixed * mid < target) a = mid + 1;
+      else b = mid;
+    }
+    return a;
+  };
+  const int64_t s_lo = bound(work * cta / NC);
+  const int64_t s_hi = cta == NC - 1 ? ns : bound(work * (cta + 1) / NC);
+  const int64_t lo = min(s_lo * 32, P.n_rows) * D, hi = min(s_hi * 32, P.n_rows) * D;
+  long long iters = c->iters;
+  const long long max_iter = c->max_iter;
+  const double tol2 = c->tol2_lo;
+  GridSync sync;
+  grid_sync_init(sync, P.sync);
+  int ref1 = 0, ref2 = 0;
+  if (threadIdx.x == 0) sh_rz = c->rz;
+  __syncthreads();
+  while (true) {
+    // ---- q = A p on own rows, partial p.q
+    DotAcc<double> pq[1];
+    int buf = 0;
+    for (int64_t base = s_lo; base < s_hi; base += NG) {
+      const int64_t s = base + grp;
+      double acc[D];
+#pragma unroll
+      for (int i = 0; i < D; ++i) acc[i] = 0.0;
+      if (s < s_hi) {
+        const int64_t b0 = P.row_ptr[s];
+        const int len = (int)((P.row_ptr[s + 1] - b0) >> 5);
+        const int32_t* cp = P.col + b0 + lane;
+        const double* vp = val + b0 * DD + lane;
+#pragma unroll (D == 1 ? 8 : D == 2 ? 4 : 2)
+        for (int k = kofs; k < len; k += KS) {
+          const int64_t cc = ld_l2(cp + (int64_t)k * 32, stream);
+          const double* vk = vp + (int64_t)k * DD * 32;
+          double m[DD], xv[D];
+#pragma unroll
+          for (int e = 0; e < DD; ++e) m[e] = ld_l2(vk + e * 32, stream);
+#pragma unroll
+          for (int j = 0; j < D; ++j) xv[j] = p[cc * D + j];
+#pragma unroll
+          for (int i = 0; i < D; ++i)
+#pragma unroll
+            for (int j = 0; j < D; ++j) acc[i] = fma(m[i * D + j], xv[j], acc[i]);
+        }
+      }
+      const int64_t a = s * 32 + lane;
+      if constexpr (KS == 1) {
+        if (s < s_hi && a < P.n_rows) {
+#pragma unroll
+          for (int i = 0; i < D; ++i) {
+            q[a * D + i] = acc[i];
+            pq[0].fma(p[a * D + i], acc[i]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < D; ++i) ys[buf][warp][i][lane] = acc[i];
+        asm volatile("barrier.sync %0, %1;" ::"r"(1 + grp), "n"(KS * 32) : "memory");
+        if (kofs < D && s < s_hi && a < P.n_rows) {  // a warp per component
+          double t = ys[buf][grp * KS][kofs][lane];
+#pragma unroll
+          for (int v = 1; v < KS; ++v) t += ys[buf][grp * KS + v][kofs][lane];
+          q[a * D + kofs] = t;
+          pq[0].fma(p[a * D + kofs], t);
+        }
+        buf ^= 1;  // the next slice's barrier separates this buffer's readers from its next writers
+      }
+    }
+    double share1[1], share2[2];
+    cta_partials<1, DotAcc<double>>(pq, share1, wsum);
+    if (threadIdx.x == 32) sh_inv = 1.0 / sh_rz;  // for the next beta, while warp 0 waits
+    const bool ok1 = grid_sum<1>(c, P.spin_limit, sync, share1, ref1, [&](const double* sm) {
+      const bool bad = zero_bits(sm[0]) || !finite_bits(sm[0]);
+      sh_stop = bad;
+      sh_alpha = sh_rz / sm[0];
+      if (bad && cta == 0) {
+        c->done = finite_bits(sm[0]) ? kDoneBreakdown : kDoneNonFinite;
+        c->iters = iters;
+      }
+    });
+    if (!ok1 || sh_stop) break;
+    // ---- r -= alpha q, z = M r on own rows
+    const double alpha = sh_alpha;
+    DotAcc<double> rzrr[2];
+#pragma unroll 4
+    for (int64_t i = lo + threadIdx.x; i < hi; i += kPThreads) {
+      const double rv = fma(-alpha, q[i], r[i]);
+      const double zv = dinv[i] * rv;
+      r[i] = rv;
+      z[i] = zv;
+      rzrr[0].fma(rv, zv);
+      rzrr[1].fma(rv, rv);
+    }
+    cta_partials<2, DotAcc<double>>(rzrr, share2, wsum);
+    const bool ok2 = grid_sum<2>(c, P.spin_limit, sync, share2, ref2, [&](const double* sm) {
+      const double rz_new = sm[0], rr = sm[1];
+      iters += 1;
+      int done = kDoneNo;
+      if (!finite_bits(rr) || !finite_bits(rz_new)) done = kDoneNonFinite;
+      else if (rr <= tol2) done = kDoneConverged;
+      else if (iters >= max_iter) done = kDoneMaxIter;
+      sh_stop = done != kDoneNo;
+      sh_beta = rz_new * sh_inv;
+      sh_rz = rz_new;
+      if (cta == 0) {
+        c->iters = iters;
+        c->rr = rr;
+        c->done = done;
+      }
+    });
+    const bool stop = !ok2 || sh_stop;
+    // ---- x += alpha p, p = z + beta p on own rows
+    const double beta = stop ? 0.0 : sh_beta;
+#pragma unroll 4
+    for (int64_t i = lo + threadIdx.x; i < hi; i += kPThreads) {
+      const double pv = p[i];
+      x[i] = fma(alpha, pv, x[i]);
+      p[i] = fma(beta, pv, z[i]);
+    }
+    if (stop) break;
+    if (!grid_barrier(c, P.spin_limit, sync)) break;
+  }
+  if (cta == 0 && threadIdx.x == 0 && *(volatile int*)&c->bar_error) c->done = kDoneBarrierTimeout;
+}
+
+// Per-iteration form of the same product's scalar (fem_set_cg_path(0)):
+// alpha = r.z / p.q, last CTA.
+__global__ void __launch_bounds__(256) k_dot_alpha(int64_t n, const double* __restrict__ p, const double* __restrict__ q,
+                                                   double* __restrict__ partial, Ctrl* ctrl) {
+  __shared__ double red[32];
+  if (ctrl_idle(ctrl)) return;
+  double t = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    t = fma(p[i], q[i], t);
+  t = block_sum(t, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  if (arrive_last(&ctrl->counter)) {
+    const double tot = sum_partials(partial, gridDim.x, 1, 0, red);
+    if (threadIdx.x == 0) {
+      ctrl->counter = 0;
+      if (tot == 0.0 || !isfinite(tot)) ctrl->done = isfinite(tot) ? kDoneBreakdown : kDoneNonFinite;
+      else ctrl->alpha = ctrl->rz / tot;
+    }
+  }
+}
+
+// FP64 CSR values into the sliced block layout: a warp per slice, a thread per
+// node row; padding slots and the off-diagonal entries that a node without
+// elements does not store become zeros.
+__global__ void __launch_bounds__(128) k_csr_to_sell64(int64_t n_nod, int D, const int64_t* __restrict__ nbr_ptr,
+                                                       const int64_t* __restrict__ inc_ptr,
+                                                       const int64_t* __restrict__ row_ptr,
+                                                       const double* __restrict__ val,
+                                                       const int64_t* __restrict__ sell_base,
+                                                       double* __restrict__ sval) {
+  const int lane = threadIdx.x & 31;
+  const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (s >= (n_nod + 31) >> 5) return;
+  const int64_t a = s * 32 + lane, b0 = sell_base[s];
+  const int len = (int)((sell_base[s + 1] - b0) >> 5);
+  const int deg = a < n_nod ? (int)(nbr_ptr[a + 1] - nbr_ptr[a]) : 0;
+  const bool orphan = a < n_nod && inc_ptr[a + 1] == inc_ptr[a];
+  double* out = sval + b0 * D * D + lane;
+  for (int i = 0; i < D; ++i) {
+    const double* row = val + (a < n_nod ? row_ptr[a * D + i] : 0);
+#pragma unroll 4
+    for (int k = 0; k < len; ++k)
+      for (int j = 0; j < D; ++j) {
+        double v = 0.0;
+        if (k < deg) v = orphan ? (i == j ? row[0] : 0.0) : row[(int64_t)k * D + j];
+        out[((int64_t)k * D * D + i * D + j) * 32] = v;
+      }
+  }
 }
 
 // ---------------------------------------------------- one-cluster FP64 CG ---
@@ -1529,61 +1950,6 @@ __device__ __forceinline__ bool cl_wait(uint32_t bar, uint32_t parity) {
     if (clock64() - t0 > kMbarSpin) return false;
   }
 }
-
-// Sums of K doubles per lane on the integer pipe, the same values in every
-// lane: each is aligned to its largest exponent as a 58-bit integer (five
-// bits below an FP64 mantissa, rounded to nearest), added exactly in three
-// redux words and rounded to FP64 once.  The error is at most 32 half units
-// of 2^-58 of the largest value plus that rounding, no more than five FP64
-// additions leave.  Exponents at either end of the range (and NaN,
-// infinities) take the FP64 tree.
-template <int K>
-__device__ __forceinline__ void sum_fixed(double (&v)[K]) {
-  int ex[K], e[K];
-  bool plain = true;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    ex[k] = (__double2hiint(v[k]) >> 20) & 0x7ff;
-    e[k] = (int)__reduce_max_sync(0xffffffffu, (unsigned)ex[k]);
-    plain = plain && e[k] >= 128 && e[k] <= 1990;
-  }
-  if (!plain) {
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      v[k] = __any_sync(0xffffffffu, (__double_as_longlong(v[k]) << 1) != 0) ? warp_sum(v[k]) : 0.0;
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const long long bits = __double_as_longlong(v[k]);
-    const int sh = min(e[k] - ex[k], 62);
-    unsigned long long m = ((unsigned long long)(bits & 0xfffffffffffffLL) | (1ull << 52)) << 5;
-    m = ex[k] == 0 ? 0ull : (m + ((1ull << sh) >> 1)) >> sh;
-    const long long f = bits < 0 ? -(long long)m : (long long)m;
-    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)f & 0x3fffffu);
-    const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 22) & 0x3fffffu);
-    const int hi = __reduce_add_sync(0xffffffffu, (int)(f >> 44));
-    const long long t = ((long long)hi << 44) + ((long long)mid << 22) + (long long)lo;
-    v[k] = t == 0 ? 0.0 : __longlong_as_double(__double_as_longlong((double)t) + ((long long)(e[k] - 1080) << 52));
-  }
-}
-
-// Kept out of line: an iteration calls them five times, and straight-line code
-// that runs once an iteration is fetched more slowly than it executes.
-__device__ __noinline__ double warp_sum_fixed(double a) {
-  double v[1] = {a};
-  sum_fixed<1>(v);
-  return v[0];
-}
-__device__ __noinline__ double2 warp_sum_fixed2(double a, double b) {
-  double v[2] = {a, b};
-  sum_fixed<2>(v);
-  return make_double2(v[0], v[1]);
-}
-
-// isfinite and == 0 by the bits: a comparison costs an FP64 instruction.
-__device__ __forceinline__ bool finite_bits(double v) { return ((__double2hiint(v) >> 20) & 0x7ff) != 0x7ff; }
-__device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
 
 // Sum of the n shares that the cluster's warps sent, on one warp.
 __device__ __forceinline__ double cl_total(const double* part, int n) {
@@ -2085,9 +2451,11 @@ __global__ void __launch_bounds__(256) k_mr_update(int64_t n, double* __restrict
 // Diagnostic for the bounded waits: CTA 1 leaves at once, CTA 0 waits at a
 // grid barrier of two CTAs that therefore never completes; the wait must run
 // out after spin_limit cycles, set bar_error and return.
-__global__ void k_diag_barrier(Ctrl* c, long long spin_limit) {
+__global__ void k_diag_barrier(Ctrl* c, unsigned long long* mem, long long spin_limit) {
   if (blockIdx.x != 0) return;
-  grid_barrier<0>(c, spin_limit, nullptr, 0, [](const double*) {});
+  GridSync sync;
+  grid_sync_init(sync, mem);
+  grid_barrier(c, spin_limit, sync);
 }
 
 // ------------------------------------------------------------- host driver --
@@ -2139,7 +2507,7 @@ static int read_ctrl(Ctrl* d, Ctrl* h, cudaStream_t st) {
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 static int64_t spmv_grid(const fem_matrix* A) {
-  if (A->format == FEM_FMT_CSR_F64) return grid_for(A->n_rows * kCsrTpr, kThreads);
+  if (A->format != FEM_FMT_SELL_F32) return grid_for(A->n_rows * kCsrTpr, kThreads);
   return sell_grid(A->n_rows);
 }
 
@@ -2156,7 +2524,7 @@ static int persistent_blocks() {
             cudaSuccess ||
         occ < 1)
       occ = 1;
-    blocks = occ * sm_count();
+    blocks = std::min(occ * sm_count(), 500);  // grid_sum counts to 511
   }
   return blocks;
 }
@@ -2173,6 +2541,10 @@ static bool use_tma_spmv() {
 
 // Upper bound on the persistent grid (at most 2048 / kPThreads CTAs per SM).
 static int64_t persistent_grid_bound() { return (int64_t)sm_count() * (2048 / kPThreads); }
+
+// GridSync memory of a grid: its counters and, per CTA, two buffers of two
+// 16-byte plain slots.
+static size_t sync_bytes(int64_t grid) { return sizeof(unsigned long long) * (kSumHead + 8 * (size_t)grid); }
 
 static int g_cg_path = -1;  // 1 persistent, 0 per-iteration kernels
 static thread_local bool g_persistent_refused = false;
@@ -2210,6 +2582,11 @@ static int validate_matrix(const fem_matrix* A) {
   if (A->format == FEM_FMT_CSR_F64) {
     if (A->block != 1 || A->n_rows != A->n) {
       set_last_error("fem_pcg: CSR needs block 1 and n_rows == n");
+      return FEM_INVALID;
+    }
+  } else if (A->format == FEM_FMT_SELL_F64) {
+    if (A->block < 1 || A->block > 3 || A->n_rows * A->block != A->n) {
+      set_last_error("fem_pcg: FP64 sliced blocks need block 1, 2 or 3 and n_rows * block == n");
       return FEM_INVALID;
     }
   } else if (A->format == FEM_FMT_SELL_F32) {
@@ -2256,13 +2633,18 @@ struct SpmvTimer {
 
 static thread_local SpmvTimer g_timer;
 
+int sell_apply64(const fem_matrix* A32, const double* sval64, const double* x, double* y, cudaStream_t st);
+
 // One CG iteration (SpMV, update, direction) on the working precision;
 // slot >= 0 brackets the SpMV with the timer's events.
 template <int G, typename VT>
 static void launch_iteration(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT* q, double* partial,
                              Ctrl* ctrl, cudaStream_t st, int slot = -1) {
   if (slot >= 0) cudaEventRecord(g_timer.ev[2 * slot], st);
-  if constexpr (G == 1) {
+  if (A->format == FEM_FMT_SELL_F64) {
+    sell_apply64(A, (const double*)A->val, (const double*)p, (double*)q, st);
+    k_dot_alpha<<<vec_grid(A->n), kThreads, 0, st>>>(A->n, (const double*)p, (const double*)q, partial, ctrl);
+  } else if constexpr (G == 1) {
     k_spmv_csr<kCsrTpr><<<grid_for(A->n_rows * kCsrTpr, kThreads), kThreads, 0, st>>>(
         A->n_rows, A->row_ptr, A->col, (const double*)A->val, (const double*)p, (double*)q,
         partial, ctrl, l2_keep_bytes() / 12);
@@ -2280,9 +2662,26 @@ static void launch_iteration(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT
   ::tfg::note_launch();
 }
 
+// A warp per slice saves the shared-memory sums, but needs slices enough to
+// load a CTA's four FP64 units evenly; below that four warps share a slice.
+// Measured (us an iteration, a warp / four warps): 3x3 blocks, 1,211 slices
+// 30.5 / 31.0, 2,154 53.4 / 45.5, 4,653 78.7 / 86.8, 11,185 180 / 196; 2x2
+// blocks, 161 slices 8.8 / 8.1, 635 9.0 / 10.1, 7,689 34.6 / 45.8; scalar rows,
+// 319 slices 8.1 / 7.8, 931 12.5 / 15.4, 7,844 19.3 / 35.4.
+template <int D>
+static cudaError_t launch_sell64(PersistParams& P, cudaStream_t st) {
+  const int64_t ns = (P.n_rows + 31) / 32;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count(), ns));
+  const void* kernel = ns >= (D == 3 ? 24 : 4) * (int64_t)grid ? (const void*)k_pcg_sell64<D, 1>
+                                                              : (const void*)k_pcg_sell64<D, 4>;
+  void* args[] = {&P};
+  cudaMemsetAsync(P.sync, 0, sync_bytes(grid), st);
+  return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kPThreads), args, 0, st);
+}
+
 // One cooperative launch of the persistent CG kernel on the given vectors.
 template <int G, typename VT>
-static int launch_persistent(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT* q, double* partial,
+static int launch_persistent(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT* q, unsigned long long* sync,
                              Ctrl* ctrl, cudaStream_t st) {
   PersistParams P;
   P.n = A->n;
@@ -2296,17 +2695,21 @@ static int launch_persistent(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT
   P.z = z;
   P.p = p;
   P.q = q;
-  P.partial = partial;
+  P.sync = sync;
   P.ctrl = ctrl;
   P.spin_limit = 2000000000LL;  // about one second of clock cycles
   void* args[] = {&P};
   cudaError_t e;
-  if (G == 3 && use_tma_spmv()) {
+  if (A->format == FEM_FMT_SELL_F64) {
+    e = A->block == 1 ? launch_sell64<1>(P, st) : A->block == 2 ? launch_sell64<2>(P, st) : launch_sell64<3>(P, st);
+  } else if (G == 3 && use_tma_spmv()) {
     const int blocks = persistent_blocks<G, VT, 1>();
+    cudaMemsetAsync(sync, 0, sync_bytes(blocks), st);
     e = cudaLaunchCooperativeKernel((const void*)k_pcg_persistent<G, VT, 1>, dim3(blocks), dim3(kPThreads), args,
                                     kTmaSmem, st);
   } else {
     const int blocks = persistent_blocks<G, VT, 0>();
+    cudaMemsetAsync(sync, 0, sync_bytes(blocks), st);
     e = cudaLaunchCooperativeKernel((const void*)k_pcg_persistent<G, VT, 0>, dim3(blocks), dim3(kPThreads), args,
                                     0, st);
   }
@@ -2323,17 +2726,17 @@ static int launch_persistent(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT
 // replacement: persistent kernel by default, per-iteration kernels when
 // TORCHFEM_GB300_CG=kernels.  Updates *h from the device.
 template <int G, typename VT>
-static int iterate(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT* q, double* partial, Ctrl* ctrl,
-                   Ctrl* h, bool timing, int* chunk, cudaStream_t st) {
+static int iterate(const fem_matrix* A, VT* x, VT* r, VT* z, VT* p, VT* q, double* partial, unsigned long long* sync,
+                   Ctrl* ctrl, Ctrl* h, bool timing, int* chunk, cudaStream_t st) {
   const long long before = h->iters;
   if (use_persistent() && !g_persistent_refused) {
     if (timing) cudaEventRecord(g_timer.ev[0], st);
-    int rc = launch_persistent<G, VT>(A, x, r, z, p, q, partial, ctrl, st);
+    int rc = launch_persistent<G, VT>(A, x, r, z, p, q, sync, ctrl, st);
     if (rc == FEM_COOP_TOO_LARGE) {
       // the device cannot hold the whole grid at once (shared with other
       // work): run this solve with per-iteration kernels instead
       g_persistent_refused = true;
-      return iterate<G, VT>(A, x, r, z, p, q, partial, ctrl, h, timing, chunk, st);
+      return iterate<G, VT>(A, x, r, z, p, q, partial, sync, ctrl, h, timing, chunk, st);
     }
     if (rc) return rc;
     if (timing) cudaEventRecord(g_timer.ev[1], st);
@@ -2395,7 +2798,7 @@ static int cluster_size() {
 static int cluster_pcg(const fem_matrix* A, const double* b, double* x, double rtol, int64_t max_iter, Ctrl* ctrl,
                        Ctrl* h, bool timing, bool* ran, cudaStream_t st) {
   *ran = false;
-  if (!use_persistent() || A->n > (int64_t)kClMax * kClRows) return FEM_OK;
+  if (A->format != FEM_FMT_CSR_F64 || !use_persistent() || A->n > (int64_t)kClMax * kClRows) return FEM_OK;
   const ClusterParams P = {A->n, A->row_ptr, A->col, (const double*)A->val, (const double*)A->precond, b, x, ctrl,
                            rtol * rtol, (long long)max_iter};
   const int c = cluster_size();
@@ -2434,13 +2837,14 @@ struct Vecs {
   Ctrl* ctrl;
   void *x, *r, *z, *p, *q;
   double* partial;
+  unsigned long long* sync;
   double* y64;
   double* fe;
   void* gather_ws;
 };
 
 static size_t layout(const fem_matrix* A, int64_t fe_len, Vecs* v, void* ws) {
-  const size_t vt = (A->format == FEM_FMT_CSR_F64) ? sizeof(double) : sizeof(float);
+  const size_t vt = (A->format == FEM_FMT_SELL_F32) ? sizeof(float) : sizeof(double);
   const int64_t n = A->n;
   char* base = reinterpret_cast<char*>(ws);
   size_t off = 0;
@@ -2457,6 +2861,7 @@ static size_t layout(const fem_matrix* A, int64_t fe_len, Vecs* v, void* ws) {
   t.p = take(n * vt);
   t.q = take(n * vt);
   t.partial = reinterpret_cast<double*>(take(sizeof(double) * 3 * (max_grid(A) + 1)));
+  t.sync = reinterpret_cast<unsigned long long*>(take(sync_bytes(persistent_grid_bound())));
   t.y64 = fe_len > 0 ? reinterpret_cast<double*>(take(sizeof(double) * n)) : nullptr;
   t.fe = fe_len > 0 ? reinterpret_cast<double*>(take(sizeof(double) * fe_len)) : nullptr;
   t.gather_ws = nullptr;
@@ -2502,7 +2907,7 @@ static int run_pcg(const fem_matrix* A, const double* b, double* x, double rtol,
     if (rc) return rc;
     int chunk = 8;
     while (h.done == kDoneNo) {
-      rc = iterate<G, VT>(A, xv, (VT*)v.r, (VT*)v.z, (VT*)v.p, (VT*)v.q, v.partial, v.ctrl, &h, timing,
+      rc = iterate<G, VT>(A, xv, (VT*)v.r, (VT*)v.z, (VT*)v.p, (VT*)v.q, v.partial, v.sync, v.ctrl, &h, timing,
                           &chunk, st);
       if (rc) return rc;
     }
@@ -2677,6 +3082,20 @@ int fem_assemble_sell_pair(const fem_blocks* B, const double* ke, const uint8_t*
   return check_cuda("fem_assemble_sell_pair");
 }
 
+int fem_csr_to_sell64(const fem_blocks* B, const int64_t* row_ptr, const double* val, const int64_t* sell_base,
+                      double* sval64, void* stream) {
+  if (B->dim < 1 || B->dim > 3) {
+    set_last_error("fem_csr_to_sell64: dim must be 1..3");
+    return FEM_INVALID;
+  }
+  if (B->n_nod == 0) return FEM_OK;
+  const int64_t ns = (B->n_nod + 31) / 32;
+  k_csr_to_sell64<<<grid_for(ns * 32, 128), 128, 0, as_stream(stream)>>>(B->n_nod, B->dim, B->nbr_ptr, B->inc_ptr,
+                                                                         row_ptr, val, sell_base, sval64);
+  ::tfg::note_launch();
+  return check_cuda("fem_csr_to_sell64");
+}
+
 int fem_sell_apply64(const fem_matrix* A32, const double* sval64, const double* x, double* y, void* stream) {
   if (!A32 || A32->format != FEM_FMT_SELL_F32 || !sval64) {
     set_last_error("fem_sell_apply64: needs the FP32 sliced matrix's layout and its FP64 copy");
@@ -2719,7 +3138,7 @@ int fem_pcg(const fem_matrix* A, const double* b, double* x, double rtol, int64_
   Vecs v;
   layout(A, 0, &v, ws);
   const bool timing = g_timing != 0;
-  if (A->format == FEM_FMT_CSR_F64) return run_pcg<1, double>(A, b, x, rtol, max_iter, v, info, st, timing);
+  if (A->format != FEM_FMT_SELL_F32) return run_pcg<1, double>(A, b, x, rtol, max_iter, v, info, st, timing);
   if (A->block == 2) return run_pcg<2, float>(A, b, x, rtol, max_iter, v, info, st, timing);
   return run_pcg<3, float>(A, b, x, rtol, max_iter, v, info, st, timing);
 }
@@ -2856,8 +3275,8 @@ int fem_pcg_mixed(const fem_matrix* A, const fem_operator64* op, const double* b
       }
       continue;
     }
-    if (G == 2) rc = iterate<2, float>(A, xl, r, z, p, q, v.partial, v.ctrl, &h, timing, &chunk, st);
-    else rc = iterate<3, float>(A, xl, r, z, p, q, v.partial, v.ctrl, &h, timing, &chunk, st);
+    if (G == 2) rc = iterate<2, float>(A, xl, r, z, p, q, v.partial, v.sync, v.ctrl, &h, timing, &chunk, st);
+    else rc = iterate<3, float>(A, xl, r, z, p, q, v.partial, v.sync, v.ctrl, &h, timing, &chunk, st);
     if (rc) return rc;
   }
   // fold whatever correction is left (max-iter exit) into x
@@ -2889,14 +3308,17 @@ int fem_pcg_mixed(const fem_matrix* A, const fem_operator64* op, const double* b
 extern "C" {
 
 int fem_diag_barrier_timeout(void* ws, size_t ws_bytes, long long spin_limit, void* stream) {
-  if (!ws || ws_bytes < sizeof(Ctrl) || spin_limit <= 0) {
-    set_last_error("fem_diag_barrier_timeout: needs a workspace of %zu bytes and a positive limit", sizeof(Ctrl));
+  if (!ws || ws_bytes < fem_diag_workspace_bytes() || spin_limit <= 0) {
+    set_last_error("fem_diag_barrier_timeout: needs a workspace of %zu bytes and a positive limit",
+                   fem_diag_workspace_bytes());
     return FEM_INVALID;
   }
   cudaStream_t st = as_stream(stream);
   Ctrl* c = reinterpret_cast<Ctrl*>(ws);
-  if (cudaMemsetAsync(c, 0, sizeof(Ctrl), st) != cudaSuccess) return check_cuda("fem_diag_barrier_timeout memset");
-  k_diag_barrier<<<2, 32, 0, st>>>(c, spin_limit);
+  if (cudaMemsetAsync(c, 0, fem_diag_workspace_bytes(), st) != cudaSuccess)
+    return check_cuda("fem_diag_barrier_timeout memset");
+  k_diag_barrier<<<2, 32, 0, st>>>(c, reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(ws) + align256(sizeof(Ctrl))),
+                                   spin_limit);
   note_launch();
   TFG_CHECK_LAUNCH("fem_diag_barrier_timeout");
   int err = 0;
@@ -2910,7 +3332,7 @@ int fem_diag_barrier_timeout(void* ws, size_t ws_bytes, long long spin_limit, vo
   return FEM_OK;
 }
 
-size_t fem_diag_workspace_bytes(void) { return sizeof(Ctrl); }
+size_t fem_diag_workspace_bytes(void) { return align256(sizeof(Ctrl)) + sync_bytes(2); }
 
 }  // extern "C"
 
@@ -3107,7 +3529,7 @@ int fem_pcg_static(const fem_matrix* A, const double* b, double* x, double rtol,
   layout(A, 0, &v, ws);
   // no SpMV event timing here: the timer creates CUDA events on first use
   // (and the process-wide timing switch is left alone)
-  if (A->format == FEM_FMT_CSR_F64) rc = run_pcg<1, double>(A, b, x, rtol, max_iter, v, info, st, false);
+  if (A->format != FEM_FMT_SELL_F32) rc = run_pcg<1, double>(A, b, x, rtol, max_iter, v, info, st, false);
   else if (A->block == 2) rc = run_pcg<2, float>(A, b, x, rtol, max_iter, v, info, st, false);
   else rc = run_pcg<3, float>(A, b, x, rtol, max_iter, v, info, st, false);
   return rc;

@@ -71,6 +71,8 @@ class LinearSystem:
         self.dm = dm
         self.precision = precision
         self.val: Tensor | None = None
+        self.cg_matrix: _lib.FemMatrix | None = None  # the form the FP64 CG runs on (DeviceMesh.cg_matrix)
+        self.cg_val: Tensor | None = None
         self.bval: Tensor | None = None
         self.bval64: Tensor | None = None
         self.precond: Tensor | None = None
@@ -580,6 +582,37 @@ class DeviceMesh:
         )
         return res, sumsq
 
+    # FP64 CG, CSR or sliced blocks.  CSR systems of up to CG_CLUSTER_NNZ[d] stored
+    # values run on the one-cluster kernel, about as fast there as the sliced
+    # grid-wide one (us an iteration, cluster / sliced: 10^3 cube, 268k values,
+    # 9.8 / 10.6; plane stress, 182k 7.7 / 8.1, 261k 9.3 / 8.2; 20^3 heat cube,
+    # 227k, 9.9 / 9.8) and ahead below.  Beyond, the sliced form is taken while its
+    # padding stores at most CG_SELL_PAD times the CSR values (Tetra1, 1.49 times:
+    # 19 against 33 us an iteration; the product's time grows with the stored slots,
+    # so at twice the values the gain would be gone).
+    CG_CLUSTER_NNZ = {1: 190_000, 2: 190_000, 3: 270_000}
+    CG_SELL_PAD = 1.6
+
+    def cg_matrix(self, sysm: LinearSystem) -> _lib.FemMatrix:
+        """The matrix of an FP64 system as its CG reads it: the CSR form, or a
+        sliced block copy of the same values."""
+        if sysm.cg_matrix is None:
+            sysm.cg_matrix = sysm.matrix
+            if self.d <= 3 and self.nnz > self.CG_CLUSTER_NNZ[self.d]:
+                base, col, n_slots = self.sell()
+                if n_slots * self.d * self.d <= self.CG_SELL_PAD * self.nnz:
+                    sysm.cg_val = self._empty(n_slots * self.d * self.d, torch.float64)
+                    check(
+                        self.lib.fem_csr_to_sell64(C.byref(self.blocks), ptr(self.row_ptr), ptr(sysm.val), ptr(base),
+                                                   ptr(sysm.cg_val), self.stream),
+                        "fem_csr_to_sell64",
+                    )
+                    sysm.cg_matrix = _lib.FemMatrix(
+                        _lib.FEM_FMT_SELL_F64, self.d, self.n_dofs, self.n_nod, ptr(base), ptr(col),
+                        ptr(sysm.cg_val), ptr(sysm.precond),
+                    )
+        return sysm.cg_matrix
+
     def solve(self, sysm: LinearSystem, b: Tensor, rtol: float, max_iter: int | None = None,
               delta: float = 0.1, refine: bool = True, linear: str = "cg") -> Tensor:
         """x with A x = b (A the condensed system), from x = 0.  For the mixed
@@ -614,8 +647,9 @@ class DeviceMesh:
                 ptr(sysm.amg_ws), sysm.amg_ws.numel(), C.byref(info), self.stream,
             )
         elif sysm.precision == "fp64" or not refine:
+            matrix = self.cg_matrix(sysm) if sysm.precision == "fp64" else sysm.matrix
             rc = self.lib.fem_pcg(
-                C.byref(sysm.matrix), ptr(b), ptr(x), rtol, max_iter, ptr(sysm.ws), sysm.ws.numel(),
+                C.byref(matrix), ptr(b), ptr(x), rtol, max_iter, ptr(sysm.ws), sysm.ws.numel(),
                 C.byref(info), self.stream,
             )
         else:

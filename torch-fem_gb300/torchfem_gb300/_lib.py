@@ -27,7 +27,7 @@ FEM_MAT_ISO, FEM_MAT_GENERAL, FEM_MAT_TANGENT_IP = 1, 2, 3
 # conductivity tensor [n_elem][dim][dim] of the heat kernels (fem_heat_*)
 FEM_MAT_CONDUCTIVITY = 16
 FEM_F64, FEM_F32 = 0, 1
-FEM_FMT_CSR_F64, FEM_FMT_SELL_F32 = 1, 2
+FEM_FMT_CSR_F64, FEM_FMT_SELL_F32, FEM_FMT_SELL_F64 = 1, 2, 3
 
 vp = C.c_void_p
 i64 = C.c_int64
@@ -238,6 +238,7 @@ _SIGNATURES = {
     "fem_sell_columns": (C.c_int, [_P(FemBlocks), vp, vp, vp]),
     "fem_assemble_sell": (C.c_int, [_P(FemBlocks), C.c_int, vp, vp, vp, i64, vp, vp]),
     "fem_assemble_sell_pair": (C.c_int, [_P(FemBlocks), vp, vp, vp, i64, vp, vp, vp]),
+    "fem_csr_to_sell64": (C.c_int, [_P(FemBlocks), vp, vp, vp, vp, vp]),
     "fem_sell_apply64": (C.c_int, [_P(FemMatrix), vp, vp, vp, vp]),
     "fem_jacobi": (C.c_int, [vp, vp, i64, vp, vp, vp]),
     "fem_block_jacobi": (C.c_int, [_P(FemBlocks), vp, vp, vp, vp, vp]),
