@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "fem_common.cuh"
+#include "fem_grid.cuh"
 
 namespace tfg {
 
@@ -972,56 +973,95 @@ __device__ __forceinline__ const float* op_operand(const OpArgs& a) {
   else return a.p;
 }
 
+// What a row's epilogue reads besides the product (the fused kernel may load it
+// before the product, so that it is there when the sums meet).
+template <int B>
+struct EpiIn {
+  float u[B], v[B], w[B], f[B], m[B * B];
+};
+template <int B, int MODE>
+__device__ __forceinline__ void epi_load(const OpArgs& a, int64_t i, EpiIn<B>& in) {
+  const int64_t o = i * B;
+#pragma unroll
+  for (int c = 0; c < B; ++c) {
+    if constexpr (MODE == kOpS1) {
+      in.u[c] = a.f[o + c];
+      in.v[c] = a.d[o + c];
+      in.w[c] = a.x[o + c];
+    } else if constexpr (MODE == kOpS2) {
+      in.u[c] = a.r[o + c];
+    } else if constexpr (MODE == kOpS3) {
+      in.u[c] = a.f[o + c];
+      in.w[c] = a.x[o + c];
+    } else if constexpr (MODE == kOpS4 || MODE == kOpS4Dot) {
+      in.u[c] = a.r[o + c];
+      in.v[c] = a.d[o + c];
+      in.w[c] = a.xb[o + c];
+      if constexpr (MODE == kOpS4Dot) in.f[c] = a.f[o + c];
+    } else if constexpr (MODE == kOpQc) {
+      in.u[c] = a.xb[o + c];
+      in.v[c] = a.p[o + c];
+      in.w[c] = a.q[o + c];
+    } else {
+      in.u[c] = a.p[o + c];
+    }
+  }
+  if constexpr (MODE == kOpS1 || MODE == kOpS3 || MODE == kOpS4 || MODE == kOpS4Dot) {
+#pragma unroll
+    for (int c = 0; c < B * B; ++c) in.m[c] = a.dinv[i * B * B + c];
+  }
+}
+
 // Row epilogue shared by the sliced and CSR kernels: y = (A v)_i; returns the
 // row's contribution to the kernel's dot product.
 template <int B, int MODE>
-__device__ __forceinline__ double op_epilogue(const OpArgs& a, int64_t i, const float (&y)[B]) {
+__device__ __forceinline__ double op_epilogue(const OpArgs& a, int64_t i, const float (&y)[B], float beta,
+                                              const EpiIn<B>& in) {
   const int64_t o = i * B;
   float t[B], rn[B];
   double dot = 0.0;
   if constexpr (MODE == kOpS1) {
 #pragma unroll
-    for (int c = 0; c < B; ++c) rn[c] = a.f[o + c] - y[c];
-    block_mv<B>(a.dinv + i * B * B, rn, t);
+    for (int c = 0; c < B; ++c) rn[c] = in.u[c] - y[c];
+    block_mv<B>(in.m, rn, t);
 #pragma unroll
     for (int c = 0; c < B; ++c) {
-      const float dn = a.c1 * a.d[o + c] + a.c2 * t[c];
+      const float dn = a.c1 * in.v[c] + a.c2 * t[c];
       a.r[o + c] = rn[c];
       a.db[o + c] = dn;
-      a.x[o + c] += dn;
+      a.x[o + c] = in.w[c] + dn;
     }
   } else if constexpr (MODE == kOpS2) {
 #pragma unroll
-    for (int c = 0; c < B; ++c) a.r[o + c] -= y[c];
+    for (int c = 0; c < B; ++c) a.r[o + c] = in.u[c] - y[c];
   } else if constexpr (MODE == kOpS3) {
 #pragma unroll
-    for (int c = 0; c < B; ++c) rn[c] = a.f[o + c] - y[c];
-    block_mv<B>(a.dinv + i * B * B, rn, t);
+    for (int c = 0; c < B; ++c) rn[c] = in.u[c] - y[c];
+    block_mv<B>(in.m, rn, t);
 #pragma unroll
     for (int c = 0; c < B; ++c) {
       const float dn = a.theta_inv * t[c];
       a.r[o + c] = rn[c];
       a.d[o + c] = dn;
-      a.xb[o + c] = a.x[o + c] + dn;
+      a.xb[o + c] = in.w[c] + dn;
     }
   } else if constexpr (MODE == kOpS4 || MODE == kOpS4Dot) {
 #pragma unroll
-    for (int c = 0; c < B; ++c) rn[c] = a.r[o + c] - y[c];
-    block_mv<B>(a.dinv + i * B * B, rn, t);
+    for (int c = 0; c < B; ++c) rn[c] = in.u[c] - y[c];
+    block_mv<B>(in.m, rn, t);
 #pragma unroll
     for (int c = 0; c < B; ++c) {
-      const float z = a.xb[o + c] + (a.c1 * a.d[o + c] + a.c2 * t[c]);
+      const float z = in.w[c] + (a.c1 * in.v[c] + a.c2 * t[c]);
       a.xb[o + c] = z;
-      if constexpr (MODE == kOpS4Dot) dot += (double)a.f[o + c] * (double)z;
+      if constexpr (MODE == kOpS4Dot) dot += (double)in.f[c] * (double)z;
     }
   } else if constexpr (MODE == kOpQc) {
     // direction update folded into the product: p = z + beta p and
     // q = A z + beta q, which carries A p by recurrence between restarts
-    const float beta = (float)a.ctrl->beta;
 #pragma unroll
     for (int c = 0; c < B; ++c) {
-      const float pn = a.xb[o + c] + beta * a.p[o + c];
-      const float qn = y[c] + beta * a.q[o + c];
+      const float pn = in.u[c] + beta * in.v[c];
+      const float qn = y[c] + beta * in.w[c];
       a.p[o + c] = pn;
       a.q[o + c] = qn;
       dot += (double)pn * (double)qn;
@@ -1030,10 +1070,18 @@ __device__ __forceinline__ double op_epilogue(const OpArgs& a, int64_t i, const 
 #pragma unroll
     for (int c = 0; c < B; ++c) {
       a.q[o + c] = y[c];
-      dot += (double)a.p[o + c] * (double)y[c];
+      dot += (double)in.u[c] * (double)y[c];
     }
   }
   return dot;
+}
+
+// beta of the direction update that kOpQc folds into its product.
+template <int B, int MODE>
+__device__ __forceinline__ double op_epilogue(const OpArgs& a, int64_t i, const float (&y)[B]) {
+  EpiIn<B> in;
+  epi_load<B, MODE>(a, i, in);
+  return op_epilogue<B, MODE>(a, i, y, MODE == kOpQc ? (float)a.ctrl->beta : 0.f, in);
 }
 
 // Only an exact zero or a non-finite value stops the iteration, as in the
@@ -1961,18 +2009,17 @@ struct CycArgs {
   CycBarrier* bar;
 };
 
-// Grid barrier with a bounded wait: one monotonic 64-bit arrival counter per
-// solve, release add by thread 0 of each CTA after a CTA barrier (cumulative:
-// it publishes the CTA's writes), relaxed polling with a short sleep, one
-// acquire fence.  A wait that runs out sets the error flag and the CG's
-// done code; returns false on every thread once any CTA's wait ran out.
-// Grid barrier of the fused cycle.  The counter only grows (it is zeroed
-// once per solve), so every barrier of a launch has a known target: the
-// first one learns the launch's base from the value its atomic returns, the
-// later ones arrive with a fire-and-forget release reduction (no round trip)
-// and poll for base + (j + 1) x grid.  `next` (thread 0's copy) carries the
-// target of the next barrier.  The wait is bounded (kCycSpin cycles); a
-// timeout flags the barrier and the solve.
+// Grid barrier of the fused cycle with a bounded wait (kCycSpin cycles; a
+// timeout flags the barrier and the solve, and the other CTAs' own waits run
+// out too).  One monotonic 64-bit arrival counter per solve: thread 0 of each
+// CTA arrives with a release after a CTA barrier (cumulative: it publishes the
+// CTA's writes) and polls with acquire loads, nothing else on the path (2,500
+// cycles on 152 CTAs; with a second load per poll, sleeps and a fence behind
+// it, 3,500 to 4,000).  The counter only grows (it is zeroed once per solve),
+// so every barrier of a launch has a known target: the first one learns the
+// launch's base from the value its atomic returns, the later ones arrive with a
+// fire-and-forget reduction.  `next` (thread 0's copy) carries the target of
+// the next barrier.
 __device__ __forceinline__ bool cyc_barrier(CycBarrier* b, AmgCtrl* c, unsigned long long& next) {
   __shared__ int ok;
   __syncthreads();
@@ -1991,21 +2038,15 @@ __device__ __forceinline__ bool cyc_barrier(CycBarrier* b, AmgCtrl* c, unsigned 
     int good = 1;
     while (true) {
       unsigned long long now;
-      asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(now) : "l"(&b->seq) : "memory");
+      asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(now) : "l"(&b->seq) : "memory");
       if (now >= target) break;
-      if (*(volatile int*)&b->error) {
-        good = 0;
-        break;
-      }
       if (clock64() - t0 > kCycSpin) {
         atomicExch(&b->error, 1);
         atomicExch(&c->done, kBarrierTimeout);
         good = 0;
         break;
       }
-      __nanosleep(32);
     }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
     ok = good;
   }
   __syncthreads();
@@ -2018,7 +2059,7 @@ template <int K, int MODE>
 __device__ __forceinline__ void cyc_row(const CycLevel& L, int64_t i, int lane, uint64_t pol) {
   constexpr int PB = 32 / K;  // blocks per pass
   constexpr int U = 2;        // passes with loads in flight together
-  const float* __restrict__ v = MODE == kOpS1 || MODE == kOpS4 ? L.d : MODE == kOpS2 ? L.db : L.x;
+  const float* v = MODE == kOpS1 || MODE == kOpS4 ? L.d : MODE == kOpS2 ? L.db : L.x;  // of other CTAs too
   const int blk = lane / K, r = lane - (lane / K) * K;
   float y = 0.f;
   if (blk < PB) {
@@ -2113,38 +2154,57 @@ __device__ __forceinline__ void cyc_restrict(const CycLevel& F, const CycLevel& 
   }
 }
 
-// Restriction onto the coarsest level and its dense solve, by one CTA.
+// Restriction onto the coarsest level and its dense solve, by one CTA: groups
+// of kGroup lanes per coarse row, so that a CTA's threads cover the level's rows
+// at once (a warp per row walked up to six rows one after the other), then a
+// warp per row of the inverse, its lanes reading it in order.
+template <int BF, int K, int kGroup>
+__device__ __forceinline__ void cyc_restrict_group(const CycLevel& F, const CycLevel& C, float* fs) {
+  const int sub = threadIdx.x % kGroup;
+  for (int64_t I0 = 0; I0 < C.n; I0 += kCycT / kGroup) {
+    const int64_t I = I0 + threadIdx.x / kGroup;
+    float acc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = 0.f;
+    if (I < C.n) {
+      const int64_t e1 = F.pt_ptr[I + 1];
+#pragma unroll 4
+      for (int64_t e = F.pt_ptr[I] + sub; e < e1; e += kGroup) {
+        const int64_t i = F.pt_row[e];
+        float pv[BF * K];
+        load_half<BF * K>(F.pt_val + e * BF * K, pv);
+#pragma unroll
+        for (int q = 0; q < BF; ++q) {
+          const float rv = F.r[i * BF + q];
+#pragma unroll
+          for (int k = 0; k < K; ++k) acc[k] = fmaf(pv[q * K + k], rv, acc[k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+      for (int o = kGroup / 2; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o, kGroup);
+      if (I < C.n && sub == 0) fs[I * K + k] = acc[k];
+    }
+  }
+}
+
 template <int BF, int K>
 __device__ __forceinline__ void cyc_coarsest(const CycLevel& F, const CycLevel& C, const float* __restrict__ inv,
                                              float* fs) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int64_t I = w; I < C.n; I += kCycT / 32) {
-    float acc[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.f;
-    for (int64_t e = F.pt_ptr[I] + lane; e < F.pt_ptr[I + 1]; e += 32) {
-      const int64_t i = F.pt_row[e];
-      float pv[BF * K];
-      load_half<BF * K>(F.pt_val + e * BF * K, pv);
-#pragma unroll
-      for (int q = 0; q < BF; ++q) {
-        const float rv = F.r[i * BF + q];
-#pragma unroll
-        for (int k = 0; k < K; ++k) acc[k] = fmaf(pv[q * K + k], rv, acc[k]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = warp_sum(acc[k]);
-    if (lane == 0)
-#pragma unroll
-      for (int k = 0; k < K; ++k) fs[I * K + k] = acc[k];
-  }
+  if (C.n > kCycT / 32) cyc_restrict_group<BF, K, 8>(F, C, fs);
+  else cyc_restrict_group<BF, K, 32>(F, C, fs);
   __syncthreads();
   const int m = (int)(C.n * K);
-  for (int t = threadIdx.x; t < m; t += kCycT) {
+  for (int t = w; t < m; t += kCycT / 32) {
     float s = 0.f;
-    for (int j = 0; j < m; ++j) s = fmaf(inv[(int64_t)t * m + j], fs[j], s);
-    C.xb[t] = s;
+#pragma unroll
+    for (int j0 = 0; j0 < kCoarseMaxDof; j0 += 32)
+      if (j0 + lane < m) s = fmaf(inv[t * m + j0 + lane], fs[j0 + lane], s);
+    s = warp_sum(s);
+    if (lane == 0) C.xb[t] = s;
   }
 }
 
@@ -2153,7 +2213,7 @@ __device__ __forceinline__ void cyc_coarsest(const CycLevel& F, const CycLevel& 
 // (every item still sums its blocks in ascending order).
 constexpr int kProlongU = 4;
 template <int BF, int K>
-__device__ __forceinline__ void cyc_prolong(const CycLevel& F, const float* __restrict__ xc, float* __restrict__ x,
+__device__ __forceinline__ void cyc_prolong(const CycLevel& F, const float* xc, float* x,
                                             int64_t t0, int64_t stride) {
   const int64_t n = F.n * BF;
   for (int64_t t = t0; t < n; t += kProlongU * stride) {
@@ -2209,7 +2269,7 @@ template <int K, int MODE>
 __device__ __forceinline__ void cyc_row_cta(const CycLevel& L, int64_t i, uint64_t pol, float* part) {
   constexpr int PB = kCycT / K;
   const int t = threadIdx.x;
-  const float* __restrict__ v = MODE == kOpS1 || MODE == kOpS4 ? L.d : MODE == kOpS2 ? L.db : L.x;
+  const float* v = MODE == kOpS1 || MODE == kOpS4 ? L.d : MODE == kOpS2 ? L.db : L.x;  // of other CTAs too
   const int blk = t / K, r = t - (t / K) * K;
   float y = 0.f;
   if (blk < PB) {
@@ -2315,14 +2375,12 @@ __device__ __forceinline__ void cyc_level_pass(const CycLevel& L, int lane, int6
   }
 }
 
+// The phases of the cycle; false once a barrier's wait ran out.  fs and part
+// are scratch, next the target of the next grid barrier (thread 0).
 template <int B0, int K>
-__global__ void __launch_bounds__(kCycT) k_coarse_cycle(CycArgs a) {
-  __shared__ float fs[kCoarseMaxDof];
-  __shared__ float part[kCycT];
+__device__ __forceinline__ bool coarse_phases(const CycArgs& a, unsigned long long& next, float* fs, float* part) {
   AmgCtrl* c = a.ctrl;
   CycBarrier* bar = a.bar;
-  if (amg_idle(c)) return;
-  unsigned long long next = 0;  // target of the next grid barrier (thread 0)
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * kCycT + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * kCycT) >> 5;
@@ -2353,27 +2411,37 @@ __global__ void __launch_bounds__(kCycT) k_coarse_cycle(CycArgs a) {
         else cyc_restrict<K, K>(F, C, I, lane);
       }
     }
-    if (!cyc_barrier(bar, c, next)) return;
+    if (!cyc_barrier(bar, c, next)) return false;
     cyc_level_pass<K, kOpS1>(C, lane, warp, n_warps, pol, part);
-    if (!cyc_barrier(bar, c, next)) return;
+    if (!cyc_barrier(bar, c, next)) return false;
     cyc_level_pass<K, kOpS2>(C, lane, warp, n_warps, pol, part);
-    if (!cyc_barrier(bar, c, next)) return;
+    if (!cyc_barrier(bar, c, next)) return false;
   }
   // up: prolongate, then the level's post-smoothing; level 0 continues in
   // the next launch
   for (int l = last - 1; l >= 0; --l) {
-    if (!cyc_barrier(bar, c, next)) return;
+    if (!cyc_barrier(bar, c, next)) return false;
     const CycLevel& F = a.L[l];
     if (l == 0) {
       cyc_prolong<B0, K>(F, a.L[1].xb, F.x, tid, n_threads);
       break;
     }
     cyc_prolong<K, K>(F, a.L[l + 1].xb, F.x, tid, n_threads);
-    if (!cyc_barrier(bar, c, next)) return;
+    if (!cyc_barrier(bar, c, next)) return false;
     cyc_level_pass<K, kOpS3>(F, lane, warp, n_warps, pol, part);
-    if (!cyc_barrier(bar, c, next)) return;
+    if (!cyc_barrier(bar, c, next)) return false;
     cyc_level_pass<K, kOpS4>(F, lane, warp, n_warps, pol, part);
   }
+  return true;
+}
+
+template <int B0, int K>
+__global__ void __launch_bounds__(kCycT) k_coarse_cycle(CycArgs a) {
+  __shared__ float fs[kCoarseMaxDof];
+  __shared__ float part[kCycT];
+  if (amg_idle(a.ctrl)) return;
+  unsigned long long next = 0;
+  coarse_phases<B0, K>(a, next, fs, part);
 }
 
 // ---------------------------------------------------------------- CG ------
@@ -2504,6 +2572,225 @@ __global__ void __launch_bounds__(256) k_cg_update(int64_t n_nod, float* __restr
       }
       if (c->done == kRun && !c->replace && c->iters >= c->max_iter) c->done = kMaxIter;
     }
+  }
+}
+
+// ------------------------------------------------ fused multigrid CG ------
+// Whole CG iterations as one cooperative launch, for systems whose level-0
+// passes are short: a launch of a few microseconds' work costs as much again in
+// launch, drain and one-CTA dot products (nine launches an iteration), a phase
+// of this kernel one grid barrier (2,500 cycles).  The phases are those of
+// launch_iteration in the same order; the level-0 passes read the matrix
+// directly, four warps to a slice of 2x2 or 3x3 blocks (as k_sell_op) or a warp
+// to a slice of scalar rows, every CTA on its own run of slices, and the dot
+// products end in grid_sum.  The CG scalars are computed by every CTA from
+// the same sums.  Runs until convergence, a due FP64 replacement or the
+// iteration limit.
+struct FusedArgs {
+  CycArgs cyc;
+  OpArgs op;  // level 0
+  int64_t n;  // nodes
+  const int64_t* sell_base;
+  const int32_t* col;
+  const float* sval;
+  float *xlo, *r;
+  unsigned long long* sync;
+};
+
+constexpr int kFusedBases = 65;  // slice bases of a CTA in shared memory
+
+// One level-0 pass over the slices [s_lo, s_hi); returns this thread's share of
+// the pass's dot product.
+template <int D, int MODE, bool H, bool kPre>
+__device__ __forceinline__ double fused_pass(const FusedArgs& g, int64_t s_lo, int64_t s_hi, float beta, float sc,
+                                             const int* base_s, float (*ys)[kCycT / 32][D][32]) {
+  constexpr int DD = D * D, KS = D > 1 ? kSellW : 1, NG = kCycT / 32 / KS;
+  const OpArgs& a = g.op;
+  const float* v = op_operand<MODE>(a);  // written by other CTAs of this launch: no __restrict__
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = warp / KS, kofs = warp % KS;
+  const uint64_t pol = l2_policy(true);
+  double dot = 0.0;
+  int buf = 0, turn = 0;
+  for (int64_t base = s_lo; base < s_hi; base += NG) {
+    const int64_t s = base + grp;
+    float y[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) y[c] = 0.f;
+    const int64_t i = s * 32 + lane;
+    const bool mine = (KS == 1 || kofs == turn) && s < s_hi && i < g.n;
+    EpiIn<D> in;
+    if (kPre && mine) epi_load<D, MODE>(a, i, in);
+    if (s < s_hi) {
+      // the CTA's first slice bases are kept in shared memory
+      const int at = (int)(s - s_lo);
+      int64_t b0;
+      int len;
+      if (at + 1 < kFusedBases) {
+        b0 = (int64_t)base_s[at] * 32;
+        len = base_s[at + 1] - base_s[at];
+      } else {
+        b0 = g.sell_base[s];
+        len = (int)((g.sell_base[s + 1] - b0) >> 5);
+      }
+      const int32_t* cp = g.col + b0 + lane;
+      const float* vp = g.sval + b0 * DD + lane;
+      const __half* hp = H ? a.sv16 + b0 * DD : nullptr;
+#pragma unroll(D == 1 ? 8 : D == 2 ? 4 : 2)
+      for (int k = kofs; k < len; k += KS) {
+        const int cc = ld_l2(cp + k * 32, pol);
+        float m[DD], xv[D];
+        load_slot<DD, H>(vp, hp, k, lane, pol, m);
+#pragma unroll
+        for (int j = 0; j < D; ++j) xv[j] = v[(int64_t)cc * D + j];
+#pragma unroll
+        for (int r = 0; r < D; ++r)
+#pragma unroll
+          for (int j = 0; j < D; ++j) y[r] = fmaf(m[r * D + j], xv[j], y[r]);
+      }
+    }
+    if constexpr (KS == 1) {
+      if (mine) {
+        if (!kPre) epi_load<D, MODE>(a, i, in);
+        y[0] = H ? y[0] * sc : y[0];
+        dot += op_epilogue<D, MODE>(a, i, y, beta, in);
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < D; ++c) ys[buf][warp][c][lane] = y[c];
+      asm volatile("barrier.sync %0, %1;" ::"r"(1 + grp), "n"(KS * 32) : "memory");
+      // the warps of a group take turns with the rows' epilogues
+      if (mine) {
+        if (!kPre) epi_load<D, MODE>(a, i, in);
+        float yt[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+          float t = ys[buf][grp * KS][c][lane];
+#pragma unroll
+          for (int u = 1; u < KS; ++u) t += ys[buf][grp * KS + u][c][lane];
+          yt[c] = H ? t * sc : t;
+        }
+        dot += op_epilogue<D, MODE>(a, i, yt, beta, in);
+      }
+      buf ^= 1;
+      turn = (turn + 1) % KS;
+    }
+  }
+  return dot;
+}
+
+// Sum of a double over the CTA, on every lane of warp 0; synchronises the CTA.
+__device__ __forceinline__ double fused_cta_sum(double v, double* wsum) {
+  v = warp_sum_fixed(v);
+  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) v = warp_sum_fixed(threadIdx.x < kCycT / 32 ? wsum[threadIdx.x] : 0.0);
+  return v;
+}
+
+template <int D, int K, bool H, int kPerSm>
+__global__ void __launch_bounds__(kCycT, kPerSm) k_amg_cg(FusedArgs g) {
+  __shared__ float fs[kCoarseMaxDof];
+  __shared__ float part[kCycT];
+  __shared__ float ys[2][kCycT / 32][D][32];
+  __shared__ int base_s[kFusedBases];
+  __shared__ double wsum[kCycT / 32];
+  __shared__ float sh_coef;
+  __shared__ int sh_stop;
+  constexpr bool kPre = kPerSm == 1;
+  AmgCtrl* c = g.cyc.ctrl;
+  if (amg_idle(c)) return;
+  const int64_t ns = (g.n + 31) >> 5;
+  const int64_t s_lo = ns * blockIdx.x / gridDim.x, s_hi = ns * (blockIdx.x + 1) / gridDim.x;
+  const int64_t lo = min(s_lo * 32, g.n), hi = min(s_hi * 32, g.n);
+  const float sc = H ? *g.op.s16inv : 1.f;  // a power of two: exact
+  GridSync sync;
+  grid_sync_init(sync, g.sync);
+  int ref_rz = 0, ref_pq = 0, ref_rr = 0;
+  int* err = &g.cyc.bar->error;
+  unsigned long long next = 0;  // thread 0: target of the next barrier
+  // CG scalars, on thread 0
+  double rz = c->rz, pscale = c->pscale, beta = 0.0, alpha = 0.0, rr = c->rr;
+  long long iters = c->iters;
+  const long long max_iter = c->max_iter;
+  const double tol2 = c->tol2_lo, delta2 = c->delta2, rr_ref = c->rr_ref;
+  const int mixed = c->mixed;
+  int done = kRun, replace = 0;
+  if (threadIdx.x == 0) sh_stop = 0;
+  if (threadIdx.x < kFusedBases && s_lo + threadIdx.x <= s_hi)
+    base_s[threadIdx.x] = (int)(g.sell_base[s_lo + threadIdx.x] >> 5);
+  __syncthreads();
+  bool ok = true;
+  while (true) {
+    // ---- z = V-cycle of r; beta
+    fused_pass<D, kOpS1, H, kPre>(g, s_lo, s_hi, 0.f, sc, base_s, ys);
+    if (!(ok = cyc_barrier(g.cyc.bar, c, next))) break;
+    fused_pass<D, kOpS2, H, kPre>(g, s_lo, s_hi, 0.f, sc, base_s, ys);
+    if (g.cyc.n_levels > 1) {
+      if (!(ok = cyc_barrier(g.cyc.bar, c, next))) break;
+      if (!(ok = coarse_phases<D, K>(g.cyc, next, fs, part))) break;
+    }
+    if (!(ok = cyc_barrier(g.cyc.bar, c, next))) break;
+    fused_pass<D, kOpS3, H, kPre>(g, s_lo, s_hi, 0.f, sc, base_s, ys);
+    if (!(ok = cyc_barrier(g.cyc.bar, c, next))) break;
+    double v[1] = {fused_cta_sum(fused_pass<D, kOpS4Dot, H, kPre>(g, s_lo, s_hi, 0.f, sc, base_s, ys), wsum)};
+    ok = grid_sum<1, true>(err, kCycSpin, sync, v, ref_rz, [&](const double* t) {
+      if (!finite_bits(t[0])) done = kNonFinite;
+      else if (zero_bits(t[0])) done = kBreakdown;
+      else {
+        beta = t[0] / rz * pscale;
+        rz = t[0];
+        pscale = 1.0;
+      }
+      sh_stop = done != kRun;
+      sh_coef = (float)beta;
+    });
+    if (!ok || sh_stop) break;
+    // ---- p = z + beta p, q = A z + beta q; alpha
+    v[0] = fused_cta_sum(fused_pass<D, kOpQc, false, kPre>(g, s_lo, s_hi, sh_coef, sc, base_s, ys), wsum);
+    ok = grid_sum<1>(err, kCycSpin, sync, v, ref_pq, [&](const double* t) {
+      if (!finite_bits(t[0])) done = kNonFinite;
+      else if (zero_bits(t[0])) done = kBreakdown;
+      else alpha = rz / t[0];
+      sh_stop = done != kRun;
+      sh_coef = (float)alpha;
+    });
+    if (!ok || sh_stop) break;
+    // ---- x += alpha p, r -= alpha q, first smoothing step of the next cycle
+    const float al = sh_coef;
+    double part_rr = 0.0;
+    for (int64_t i = lo + threadIdx.x; i < hi; i += kCycT) {
+      float rv[D];
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        const int64_t o = i * D + k;
+        g.xlo[o] += al * g.op.p[o];
+        rv[k] = g.r[o] - al * g.op.q[o];
+        g.r[o] = rv[k];
+        part_rr += (double)rv[k] * (double)rv[k];
+      }
+      pre_step<D>(g.op.dinv, g.op.theta_inv, i, rv, g.op.d, g.op.x);
+    }
+    v[0] = fused_cta_sum(part_rr, wsum);
+    ok = grid_sum<1, true>(err, kCycSpin, sync, v, ref_rr, [&](const double* t) {
+      iters += 1;
+      rr = t[0];
+      if (!finite_bits(rr)) done = kNonFinite;
+      else if (mixed) replace = rr <= tol2 || rr <= delta2 * rr_ref;
+      else if (rr <= tol2) done = kConverged;
+      if (done == kRun && !replace && iters >= max_iter) done = kMaxIter;
+      sh_stop = done != kRun || replace;
+    });
+    if (!ok || sh_stop) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    c->rz = rz;
+    c->pscale = pscale;
+    c->beta = beta;
+    c->alpha = alpha;
+    c->rr = rr;
+    c->iters = iters;
+    c->replace = replace;
+    c->done = ok ? done : kBarrierTimeout;
   }
 }
 
@@ -2784,6 +3071,9 @@ struct fem_amg {
   // fused coarse cycle: CTAs (0 not yet sized, -1 unavailable) and barrier state
   int cyc_blocks = 0;
   tfg::CycBarrier* cyc_bar = nullptr;
+  // fused CG: CTAs (0 not yet sized, -1 unavailable) and its grid_sum memory
+  int cg_blocks = 0;
+  unsigned long long* cg_sync = nullptr;
 
   template <typename T>
   T* alloc(int64_t count, cudaStream_t st) {
@@ -3428,28 +3718,7 @@ void launch_coarse_levels(fem_amg* h, cudaStream_t st) {
   }
 }
 
-// The same coarse part as one cooperative launch of k_coarse_cycle.  Returns
-// false when the launch is refused (the caller then runs the per-level
-// kernels), after which the handle stops trying.
-template <int B0, int K>
-bool launch_coarse_fused(fem_amg* h, cudaStream_t st) {
-  if (h->cyc_blocks < 0) return false;
-  if (h->cyc_blocks == 0) {
-    int dev = 0, coop = 0, occ = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_coarse_cycle<B0, K>, kCycT, 0) != cudaSuccess ||
-        occ < 1) {
-      cudaGetLastError();
-      h->cyc_blocks = -1;
-      return false;
-    }
-    h->cyc_blocks = std::min(occ, kCycPerSm) * sm_count();
-    // small hierarchies: no more CTAs than level 1 has rows for their warps
-    // (each grid barrier waits for every CTA)
-    const int64_t need = (h->L[1].n + kCycT / 32 - 1) / (kCycT / 32);
-    h->cyc_blocks = (int)std::max<int64_t>(std::min<int64_t>(need, h->cyc_blocks), std::min(32, h->cyc_blocks));
-  }
+CycArgs cycle_args(const fem_amg* h) {
   CycArgs ca{};
   ca.n_levels = h->n_levels;
   for (int l = 0; l < h->n_levels; ++l) {
@@ -3479,6 +3748,32 @@ bool launch_coarse_fused(fem_amg* h, cudaStream_t st) {
   ca.coarse_inv = h->coarse_inv;
   ca.ctrl = h->ctrl;
   ca.bar = h->cyc_bar;
+  return ca;
+}
+
+// The same coarse part as one cooperative launch of k_coarse_cycle.  Returns
+// false when the launch is refused (the caller then runs the per-level
+// kernels), after which the handle stops trying.
+template <int B0, int K>
+bool launch_coarse_fused(fem_amg* h, cudaStream_t st) {
+  if (h->cyc_blocks < 0) return false;
+  if (h->cyc_blocks == 0) {
+    int dev = 0, coop = 0, occ = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_coarse_cycle<B0, K>, kCycT, 0) != cudaSuccess ||
+        occ < 1) {
+      cudaGetLastError();
+      h->cyc_blocks = -1;
+      return false;
+    }
+    h->cyc_blocks = std::min(occ, kCycPerSm) * sm_count();
+    // small hierarchies: no more CTAs than level 1 has rows for their warps
+    // (each grid barrier waits for every CTA)
+    const int64_t need = (h->L[1].n + kCycT / 32 - 1) / (kCycT / 32);
+    h->cyc_blocks = (int)std::max<int64_t>(std::min<int64_t>(need, h->cyc_blocks), std::min(32, h->cyc_blocks));
+  }
+  CycArgs ca = cycle_args(h);
 
   void* args[] = {&ca};
   if (cudaLaunchCooperativeKernel((const void*)k_coarse_cycle<B0, K>, dim3(h->cyc_blocks), dim3(kCycT), args, 0,
@@ -3514,6 +3809,69 @@ void launch_iteration(fem_amg* h, cudaStream_t st) {
   launch_chain(capped(grid_for(h->L[0].n, kT), 8), kT, 0, st, k_cg_update<B0>, h->L[0].n, h->xlo, h->rcg, h->p,
                h->q, h->dinv0, h->L[0].theta_inv, h->L[0].d, h->L[0].x, h->partial, h->ctrl);
   note_launch();
+}
+
+// CG iterations as one launch of k_amg_cg, until they stop.  Returns false where
+// the system is too large for it to pay or the launch is refused.  By the bytes
+// of a smoothing pass (FP16 values and columns): up to 16 MB one CTA per SM, with
+// registers to load a row's epilogue before its product, then two; beyond 64 MB
+// the bulk copies of the separate launches stream the matrix faster.  Measured
+// (us an iteration, launches / one CTA / two): 28^3 cube, 14 MB, 131 / 107 / 112;
+// 40^3, 40 MB, 193 / 205 / 184; 56^3, 108 MB, 330 / 432 / 323; plane stress
+// 400 x 200, 9 MB, 138 / 106 / 106; 900 x 450, 44 MB, 353 / 383 / 294; heat slab
+// 320 x 160, 11 MB, 123 / 89 / 94; 724 x 362, 57 MB, 237 / 240 / 204; 1024 x 512,
+// 114 MB, 352 / 484 / 366.
+constexpr int64_t kFusedOne = 16 << 20, kFusedMost = 64 << 20;
+template <int B0, int K>
+bool launch_fused_cg(fem_amg* h, cudaStream_t st) {
+  const int64_t slots = h->sv16_len / (B0 * B0), pass = slots * (2 * B0 * B0 + 4);
+  if (h->cg_blocks < 0 || pass > kFusedMost) return false;
+  const bool half = h->sv16 && g_amg_half;
+  const bool one = pass <= kFusedOne;
+  const void* kernel = half ? (one ? (const void*)k_amg_cg<B0, K, true, 1> : (const void*)k_amg_cg<B0, K, true, 2>)
+                            : (one ? (const void*)k_amg_cg<B0, K, false, 1> : (const void*)k_amg_cg<B0, K, false, 2>);
+  if (h->cg_blocks == 0) {
+    int dev = 0, coop = 0, occ = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kCycT, 0) != cudaSuccess || occ < 1) {
+      cudaGetLastError();
+      h->cg_blocks = -1;
+      return false;
+    }
+    // a group of warps per slice, as far as the GPU holds them
+    const int64_t ns = (h->L[0].n + 31) / 32, per = kCycT / 32 / (B0 > 1 ? kSellW : 1);
+    h->cg_blocks = (int)std::max<int64_t>(
+        1, std::min<int64_t>((ns + per - 1) / per, std::min(std::min(occ, kCycPerSm) * sm_count(), 500)));
+    h->cg_sync = h->alloc<unsigned long long>((int64_t)(sync_bytes(h->cg_blocks) / sizeof(unsigned long long)), st);
+    if (!h->cg_sync) {
+      cudaGetLastError();
+      h->cg_blocks = -1;
+      return false;
+    }
+  }
+  FusedArgs fa;
+  fa.cyc = cycle_args(h);
+  fa.op = level_args(h, 0, h->ctrl);
+  fa.op.p = h->p;
+  fa.op.q = h->q;
+  fa.n = h->L[0].n;
+  fa.sell_base = h->sell_base;
+  fa.col = h->sell_col;
+  fa.sval = h->sell_val;
+  fa.xlo = h->xlo;
+  fa.r = h->rcg;
+  fa.sync = h->cg_sync;
+  cudaMemsetAsync(h->cg_sync, 0, sync_bytes(h->cg_blocks), st);
+  cudaMemsetAsync(h->cyc_bar, 0, sizeof(CycBarrier), st);
+  void* args[] = {&fa};
+  if (cudaLaunchCooperativeKernel(kernel, dim3(h->cg_blocks), dim3(kCycT), args, 0, st) != cudaSuccess) {
+    cudaGetLastError();
+    h->cg_blocks = -1;
+    return false;
+  }
+  note_launch();
+  return true;
 }
 
 int read_ctrl(fem_amg* h, AmgCtrl* c, cudaStream_t st) {
@@ -3618,6 +3976,12 @@ int pcg_impl(fem_amg* h, const fem_matrix* A, const fem_operator64* op, const do
           return FEM_NOT_CONVERGED;
         }
       }
+      continue;
+    }
+    if (!timing && g_amg_fused && launch_fused_cg<B0, K>(h, st)) {
+      rc = check_cuda("AMG CG");
+      if (!rc) rc = read_ctrl(h, &c, st);
+      if (rc) return rc;
       continue;
     }
     const long long before = c.iters;
