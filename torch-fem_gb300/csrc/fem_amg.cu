@@ -329,13 +329,13 @@ __global__ void k_sort_rows(int64_t n_rows, const int64_t* __restrict__ ptr, con
 }
 
 // Position in P of every transposed entry: the slot of coarse column I in the
-// P row of fine node pt_row[e].
+// P row of fine node pt_row[e].  Warp per coarse row.
 __global__ void k_pt_pos(int64_t n_c, const int64_t* __restrict__ pt_ptr, const int32_t* __restrict__ pt_row,
                          const int64_t* __restrict__ p_ptr, const int32_t* __restrict__ p_col,
                          int64_t* __restrict__ pt_pos) {
-  const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t I = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (I >= n_c) return;
-  for (int64_t e = pt_ptr[I]; e < pt_ptr[I + 1]; ++e) {
+  for (int64_t e = pt_ptr[I] + (threadIdx.x & 31); e < pt_ptr[I + 1]; e += 32) {
     const int32_t i = pt_row[e];
     int64_t pos = -1;
     for (int64_t f = p_ptr[i]; f < p_ptr[i + 1]; ++f)
@@ -382,31 +382,71 @@ __global__ void k_p_rows(Graph g, const uint8_t* __restrict__ active, const int3
   }
 }
 
-// Union pattern: row i holds the union over u in outer(i) of inner(u);
-// rows of inactive nodes (active[i] == 0) stay empty.
+// Union pattern: row i holds the union over u in outer(i) of inner(u), in
+// ascending order; rows of inactive nodes (active[i] == 0) stay empty.  Warp per
+// row: its lanes take the outer entries and insert the columns into a hash set in
+// shared memory, which is then compacted and ranked.  (A thread per row with
+// sorted insertion left a coarse level's few hundred rows, thousands of columns
+// each, to as many threads: 1.2 ms a call on the 27x22x31 cube.)
+constexpr int kUnionW = 4;  // warps of a CTA
 template <int CAP, bool kFill>
-__global__ void k_union_rows(int64_t n, const uint8_t* __restrict__ active, const int64_t* __restrict__ optr,
-                             const int32_t* __restrict__ oidx, const int64_t* __restrict__ iptr,
-                             const int32_t* __restrict__ icol, int64_t* __restrict__ cnt,
-                             const int64_t* __restrict__ ptr, int32_t* __restrict__ col, int32_t* __restrict__ status) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kUnionW * 32)
+k_union_rows(int64_t n, const uint8_t* __restrict__ active, const int64_t* __restrict__ optr,
+             const int32_t* __restrict__ oidx, const int64_t* __restrict__ iptr, const int32_t* __restrict__ icol,
+             int64_t* __restrict__ cnt, const int64_t* __restrict__ ptr, int32_t* __restrict__ col,
+             int32_t* __restrict__ status) {
+  constexpr int HT = 4 * CAP;  // at most CAP + 32 columns go in: every lane checks the count first
+  static_assert((HT & (HT - 1)) == 0 && CAP + 32 < HT, "hash table size");
+  __shared__ int32_t table[kUnionW][HT];
+  __shared__ int32_t list[kUnionW][CAP];
+  __shared__ int count[kUnionW];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = (int64_t)blockIdx.x * kUnionW + w;
   if (i >= n) return;
-  int32_t s[CAP];
-  int m = 0;
-  bool ok = !active || active[i];
-  for (int64_t e = optr[i]; e < optr[i + 1] && ok; ++e) {
-    const int32_t u = oidx[e];
-    for (int64_t f = iptr[u]; f < iptr[u + 1]; ++f)
-      if (!insert_unique(s, m, icol[f])) {
-        flag_status(status, kStatBounds);
-        ok = false;
-        break;
+  for (int t = lane; t < HT; t += 32) table[w][t] = -1;
+  if (lane == 0) count[w] = 0;
+  __syncwarp();
+  if (!active || active[i]) {
+    for (int64_t e = optr[i] + lane; e < optr[i + 1]; e += 32) {
+      const int32_t u = oidx[e];
+      const int64_t f1 = iptr[u + 1];
+      for (int64_t f = iptr[u]; f < f1; ++f) {
+        const int32_t v = icol[f];
+        if (*(volatile int*)&count[w] > CAP) break;
+        int h = (int)(((uint32_t)v * 2654435769u) & (HT - 1));
+        while (true) {
+          const int32_t old = atomicCAS(&table[w][h], -1, v);
+          if (old == -1) atomicAdd(&count[w], 1);
+          if (old == -1 || old == v) break;
+          h = (h + 1) & (HT - 1);
+        }
       }
+    }
+  }
+  __syncwarp();
+  int m = count[w];
+  if (m > CAP) {
+    if (lane == 0) flag_status(status, kStatBounds);
+    m = CAP;
   }
   if (!kFill) {
-    cnt[i] = m;
-  } else {
-    for (int k = 0; k < m; ++k) col[ptr[i] + k] = s[k];
+    if (lane == 0) cnt[i] = m;
+    return;
+  }
+  int at = 0;
+  for (int t0 = 0; t0 < HT; t0 += 32) {
+    const int32_t v = table[w][t0 + lane];
+    const unsigned b = __ballot_sync(0xffffffffu, v >= 0);
+    const int k = at + __popc(b & ((1u << lane) - 1));
+    if (v >= 0 && k < CAP) list[w][k] = v;
+    at += __popc(b);
+  }
+  __syncwarp();
+  for (int k = lane; k < m; k += 32) {
+    const int32_t v = list[w][k];
+    int rank = 0;
+    for (int j = 0; j < m; ++j) rank += list[w][j] < v;
+    col[ptr[i] + rank] = v;
   }
 }
 
@@ -763,30 +803,70 @@ __global__ void __launch_bounds__(256) k_ap_numeric(int64_t n_slots, OpView<B, k
 // per contribution with all K x K products in registers, then a fixed-order
 // warp reduction.  Decoupled coarse DOFs (a dropped mode: zero row and
 // column) get a unit diagonal.
+//
+// The lists: a CTA per coarse row, its warps on consecutive runs of the row's
+// P^T entries, lanes on the columns of an entry's A P row (distinct, so their
+// blocks are).  A first walk counts per (warp, block), which gives every warp its
+// start in each list; the second writes in order.  (A thread per coarse row took
+// 1.4 and 2.1 ms on the 27x22x31 cube.)
+constexpr int kAcW = 8;
 template <bool kFill>
-__global__ void k_ac_lists(int64_t n_c, const int64_t* __restrict__ pt_ptr, const int32_t* __restrict__ pt_row,
-                           const int64_t* __restrict__ pt_pos, const int64_t* __restrict__ ap_ptr,
-                           const int32_t* __restrict__ ap_col, const int64_t* __restrict__ ac_ptr,
-                           const int32_t* __restrict__ ac_col, int64_t* __restrict__ cnt,
-                           int64_t* __restrict__ cursor, int32_t* __restrict__ cl_p, int32_t* __restrict__ cl_w) {
-  const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= n_c) return;
+__global__ void __launch_bounds__(kAcW * 32)
+k_ac_lists(const int64_t* __restrict__ pt_ptr, const int32_t* __restrict__ pt_row, const int64_t* __restrict__ pt_pos,
+           const int64_t* __restrict__ ap_ptr, const int32_t* __restrict__ ap_col, const int64_t* __restrict__ ac_ptr,
+           const int32_t* __restrict__ ac_col, int64_t* __restrict__ cnt, const int64_t* __restrict__ cl_ptr,
+           int32_t* __restrict__ cl_p, int32_t* __restrict__ cl_w) {
+  __shared__ int32_t cols[kMaxCRow];
+  __shared__ int64_t at[kAcW][kMaxCRow];
+  const int64_t I = blockIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t a0 = ac_ptr[I];
   const int m = (int)(ac_ptr[I + 1] - a0);
-  for (int64_t pe = pt_ptr[I]; pe < pt_ptr[I + 1]; ++pe) {
-    const int32_t i = pt_row[pe];
-    for (int64_t ae = ap_ptr[i]; ae < ap_ptr[i + 1]; ++ae) {
-      const int s = bsearch_slot(ac_col + a0, m, ap_col[ae]);
-      if (s < 0) continue;  // cannot happen: the row is the union of these columns
-      if (!kFill) {
-        cnt[a0 + s] += 1;
-      } else {
-        const int64_t pos = cursor[a0 + s]++;
-        cl_p[pos] = (int32_t)pt_pos[pe];
-        cl_w[pos] = (int32_t)ae;
+  for (int s = threadIdx.x; s < m; s += kAcW * 32) cols[s] = ac_col[a0 + s];
+  for (int s = threadIdx.x; s < kAcW * kMaxCRow; s += kAcW * 32) at[s / kMaxCRow][s % kMaxCRow] = 0;
+  __syncthreads();
+  const int64_t p0 = pt_ptr[I], np = pt_ptr[I + 1] - p0;
+  const int64_t lo = p0 + np * w / kAcW, hi = p0 + np * (w + 1) / kAcW;
+  auto walk = [&](auto&& visit) {
+    for (int64_t b = lo; b < hi; b += 32) {
+      // 32 entries' A P rows at a time
+      int64_t r0 = 0;
+      int len = 0;
+      if (b + lane < hi) {
+        const int32_t i = pt_row[b + lane];
+        r0 = ap_ptr[i];
+        len = (int)(ap_ptr[i + 1] - r0);
+      }
+      const int ne = (int)min((int64_t)32, hi - b);
+      for (int t = 0; t < ne; ++t) {
+        const int64_t q0 = __shfl_sync(0xffffffffu, r0, t);
+        const int n = __shfl_sync(0xffffffffu, len, t);
+        for (int k = lane; k < n; k += 32) {
+          const int s = bsearch_slot(cols, m, ap_col[q0 + k]);
+          if (s >= 0) visit(s, b + t, q0 + k);  // always: the row is the union of these columns
+        }
+        __syncwarp();
       }
     }
+  };
+  walk([&](int s, int64_t, int64_t) { at[w][s] += 1; });
+  __syncthreads();
+  for (int s = threadIdx.x; s < m; s += kAcW * 32) {
+    int64_t sum = kFill ? cl_ptr[a0 + s] : 0;
+    for (int u = 0; u < kAcW; ++u) {
+      const int64_t c = at[u][s];
+      at[u][s] = sum;
+      sum += c;
+    }
+    if (!kFill) cnt[a0 + s] = sum;
   }
+  if (!kFill) return;
+  __syncthreads();
+  walk([&](int s, int64_t pe, int64_t ae) {
+    const int64_t pos = at[w][s]++;
+    cl_p[pos] = (int32_t)pt_pos[pe];
+    cl_w[pos] = (int32_t)ae;
+  });
 }
 
 template <int B, int K>
@@ -3273,20 +3353,20 @@ int patterns(fem_amg* h, int l, cudaStream_t st) {
   note_launch();
   k_sort_rows<<<grid_for(na * 32, kT), kT, 0, st>>>(na, L.pt_ptr, unsorted, L.pt_row);
   note_launch();
-  k_pt_pos<<<grid_for(na, kT), kT, 0, st>>>(na, L.pt_ptr, L.pt_row, L.p_ptr, L.p_col, L.pt_pos);
+  k_pt_pos<<<grid_for(na * 32, kT), kT, 0, st>>>(na, L.pt_ptr, L.pt_row, L.p_ptr, L.p_col, L.pt_pos);
   note_launch();
   // A P: union of the P rows of the neighbours (rows of inactive nodes stay
   // empty: their P rows are empty and no coarse row reads them)
   L.ap_ptr = h->alloc<int64_t>(n + 1, st);
   if (!L.ap_ptr) return check_cuda("AMG AP pattern");
-  k_union_rows<kMaxAPRow, false><<<gn, kT, 0, st>>>(n, active, L.g.ptr, L.g.idx, L.p_ptr, L.p_col, cnt, nullptr,
+  k_union_rows<kMaxAPRow, false><<<grid_for(n, kUnionW), kUnionW * 32, 0, st>>>(n, active, L.g.ptr, L.g.idx, L.p_ptr, L.p_col, cnt, nullptr,
                                                      nullptr, h->status);
   note_launch();
   rc = scan_total(h, cnt, L.ap_ptr, n, &L.ap_nnz, st);
   if (rc) return rc;
   L.ap_col = h->alloc<int32_t>(L.ap_nnz, st);
   if (!L.ap_col) return check_cuda("AMG AP pattern");
-  k_union_rows<kMaxAPRow, true><<<gn, kT, 0, st>>>(n, active, L.g.ptr, L.g.idx, L.p_ptr, L.p_col, nullptr,
+  k_union_rows<kMaxAPRow, true><<<grid_for(n, kUnionW), kUnionW * 32, 0, st>>>(n, active, L.g.ptr, L.g.idx, L.p_ptr, L.p_col, nullptr,
                                                     L.ap_ptr, L.ap_col, h->status);
   note_launch();
   // coarse operator: union over the P^T row of the A P rows
@@ -3294,14 +3374,14 @@ int patterns(fem_amg* h, int l, cudaStream_t st) {
   C.b = h->K;
   C.a_ptr = h->alloc<int64_t>(na + 1, st);
   if (!C.a_ptr) return check_cuda("AMG coarse pattern");
-  k_union_rows<kMaxCRow, false><<<grid_for(na, kT), kT, 0, st>>>(na, nullptr, L.pt_ptr, L.pt_row, L.ap_ptr,
+  k_union_rows<kMaxCRow, false><<<grid_for(na, kUnionW), kUnionW * 32, 0, st>>>(na, nullptr, L.pt_ptr, L.pt_row, L.ap_ptr,
                                                                  L.ap_col, cnt, nullptr, nullptr, h->status);
   note_launch();
   rc = scan_total(h, cnt, C.a_ptr, na, &C.a_nnz, st);
   if (rc) return rc;
   C.a_col = h->alloc<int32_t>(C.a_nnz, st);
   if (!C.a_col) return check_cuda("AMG coarse pattern");
-  k_union_rows<kMaxCRow, true><<<grid_for(na, kT), kT, 0, st>>>(na, nullptr, L.pt_ptr, L.pt_row, L.ap_ptr,
+  k_union_rows<kMaxCRow, true><<<grid_for(na, kUnionW), kUnionW * 32, 0, st>>>(na, nullptr, L.pt_ptr, L.pt_row, L.ap_ptr,
                                                                 L.ap_col, nullptr, C.a_ptr, C.a_col, h->status);
   note_launch();
   C.g = Graph{na, C.a_ptr, C.a_col};
@@ -3335,12 +3415,10 @@ int patterns(fem_amg* h, int l, cudaStream_t st) {
   L.slot_row = h->alloc<int32_t>(C.a_nnz, st);
   int64_t* ccnt = h->alloc<int64_t>(C.a_nnz + 1, st);
   L.cl_ptr = h->alloc<int64_t>(C.a_nnz + 1, st);
-  int64_t* ccur = h->alloc<int64_t>(C.a_nnz + 1, st);
-  if (!L.slot_row || !ccnt || !L.cl_ptr || !ccur) return check_cuda("AMG Galerkin lists");
+  if (!L.slot_row || !ccnt || !L.cl_ptr) return check_cuda("AMG Galerkin lists");
   k_slot_rows<<<grid_for(na, kT), kT, 0, st>>>(na, C.a_ptr, L.slot_row);
   note_launch();
-  cudaMemsetAsync(ccnt, 0, sizeof(int64_t) * (C.a_nnz + 1), st);
-  k_ac_lists<false><<<grid_for(na, 128), 128, 0, st>>>(na, L.pt_ptr, L.pt_row, L.pt_pos, L.ap_ptr, L.ap_col, C.a_ptr,
+  k_ac_lists<false><<<(unsigned)na, kAcW * 32, 0, st>>>(L.pt_ptr, L.pt_row, L.pt_pos, L.ap_ptr, L.ap_col, C.a_ptr,
                                                        C.a_col, ccnt, nullptr, nullptr, nullptr);
   note_launch();
   int64_t n_cl = 0;
@@ -3353,9 +3431,8 @@ int patterns(fem_amg* h, int l, cudaStream_t st) {
   L.cl_p = h->alloc<int32_t>(n_cl, st);
   L.cl_w = h->alloc<int32_t>(n_cl, st);
   if (!L.cl_p || !L.cl_w) return check_cuda("AMG Galerkin lists");
-  cudaMemcpyAsync(ccur, L.cl_ptr, sizeof(int64_t) * (C.a_nnz + 1), cudaMemcpyDeviceToDevice, st);
-  k_ac_lists<true><<<grid_for(na, 128), 128, 0, st>>>(na, L.pt_ptr, L.pt_row, L.pt_pos, L.ap_ptr, L.ap_col, C.a_ptr,
-                                                      C.a_col, nullptr, ccur, L.cl_p, L.cl_w);
+  k_ac_lists<true><<<(unsigned)na, kAcW * 32, 0, st>>>(L.pt_ptr, L.pt_row, L.pt_pos, L.ap_ptr, L.ap_col, C.a_ptr,
+                                                      C.a_col, nullptr, L.cl_ptr, L.cl_p, L.cl_w);
   note_launch();
   return read_status(h, st, "AMG patterns");
 }
