@@ -2133,6 +2133,38 @@ __device__ __forceinline__ bool cyc_barrier(CycBarrier* b, AmgCtrl* c, unsigned 
   return ok != 0;
 }
 
+// K consecutive values, by 8-byte loads where K is even (blocks of K x K and rows
+// of K values then start on 8 bytes).
+template <int K>
+__device__ __forceinline__ void load_row(const float* src, float (&dst)[K]) {
+  if constexpr (K % 2 == 0) {
+#pragma unroll
+    for (int q = 0; q < K / 2; ++q) {
+      const float2 f = reinterpret_cast<const float2*>(src)[q];
+      dst[2 * q] = f.x;
+      dst[2 * q + 1] = f.y;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < K; ++q) dst[q] = src[q];
+  }
+}
+template <int K>
+__device__ __forceinline__ void load_row_l2(const float* src, uint64_t pol, float (&dst)[K]) {
+  if constexpr (K % 2 == 0) {
+#pragma unroll
+    for (int q = 0; q < K / 2; ++q) {
+      float2 f;
+      asm("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(f.x), "=f"(f.y) : "l"(src + 2 * q), "l"(pol));
+      dst[2 * q] = f.x;
+      dst[2 * q + 1] = f.y;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < K; ++q) dst[q] = ld_l2(src + q, pol);
+  }
+}
+
 // One Chebyshev pass of a coarse level on block row i by one warp (the
 // modes S1..S4 of op_epilogue).
 template <int K, int MODE>
@@ -2143,23 +2175,31 @@ __device__ __forceinline__ void cyc_row(const CycLevel& L, int64_t i, int lane, 
   const int blk = lane / K, r = lane - (lane / K) * K;
   float y = 0.f;
   if (blk < PB) {
-    const int64_t e1 = L.a_ptr[i + 1];
-    for (int64_t e = L.a_ptr[i] + blk; e < e1; e += U * PB) {
-      int64_t c[U];
+    // the next pass's columns load while this pass's values and gathers do
+    const int64_t e0 = L.a_ptr[i] + blk, e1 = L.a_ptr[i + 1];
+    int c[U];
 #pragma unroll
-      for (int w = 0; w < U; ++w) c[w] = e + w * PB < e1 ? (int64_t)ld_l2(L.a_col + e + w * PB, pol) : -1;
+    for (int w = 0; w < U; ++w) c[w] = e0 + w * PB < e1 ? ld_l2(L.a_col + e0 + w * PB, pol) : -1;
+    for (int64_t e = e0; e < e1; e += U * PB) {
       float m[U][K], xv[U][K];
+      int cn[U];
 #pragma unroll
-      for (int w = 0; w < U; ++w)
+      for (int w = 0; w < U; ++w) {
+        if (c[w] >= 0) {
+          load_row_l2<K>(L.a_val + (e + w * PB) * K * K + r * K, pol, m[w]);
+          load_row<K>(v + (int64_t)c[w] * K, xv[w]);
+        } else {
 #pragma unroll
-        for (int q = 0; q < K; ++q) {
-          m[w][q] = c[w] >= 0 ? ld_l2(L.a_val + (e + w * PB) * K * K + r * K + q, pol) : 0.f;
-          xv[w][q] = c[w] >= 0 ? v[c[w] * K + q] : 0.f;
+          for (int q = 0; q < K; ++q) m[w][q] = xv[w][q] = 0.f;
         }
+        cn[w] = e + (U + w) * PB < e1 ? ld_l2(L.a_col + e + (U + w) * PB, pol) : -1;
+      }
 #pragma unroll
-      for (int w = 0; w < U; ++w)
+      for (int w = 0; w < U; ++w) {
 #pragma unroll
         for (int q = 0; q < K; ++q) y = fmaf(m[w][q], xv[w][q], y);
+        c[w] = cn[w];
+      }
     }
   }
   // lane r (< K) adds the lanes r + b K, b = 1 .. PB-1, in order
@@ -2207,16 +2247,35 @@ __device__ __forceinline__ void cyc_restrict(const CycLevel& F, const CycLevel& 
   float acc[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = 0.f;
-  for (int64_t e = F.pt_ptr[I] + lane; e < F.pt_ptr[I + 1]; e += 32) {
-    const int64_t i = F.pt_row[e];
-    float pv[BF * K];
-    load_half<BF * K>(F.pt_val + e * BF * K, pv);
+  // the next entries' fine rows load while this pass's values do
+  constexpr int U = BF * K == 1 ? 4 : BF * K <= 6 ? 2 : 1;
+  const int64_t e1 = F.pt_ptr[I + 1];
+  int64_t e = F.pt_ptr[I] + lane;
+  int i[U];
 #pragma unroll
-    for (int q = 0; q < BF; ++q) {
-      const float rv = F.r[i * BF + q];
+  for (int u = 0; u < U; ++u) i[u] = e + 32 * u < e1 ? F.pt_row[e + 32 * u] : -1;
+  for (; e < e1; e += 32 * U) {
+    float pv[U][BF * K], rv[U][BF];
 #pragma unroll
-      for (int k = 0; k < K; ++k) acc[k] = fmaf(pv[q * K + k], rv, acc[k]);
+    for (int u = 0; u < U; ++u) {
+      if (i[u] >= 0) {
+        load_half<BF * K>(F.pt_val + (e + 32 * u) * BF * K, pv[u]);
+#pragma unroll
+        for (int q = 0; q < BF; ++q) rv[u][q] = F.r[(int64_t)i[u] * BF + q];
+      } else {
+#pragma unroll
+        for (int q = 0; q < BF * K; ++q) pv[u][q] = 0.f;
+#pragma unroll
+        for (int q = 0; q < BF; ++q) rv[u][q] = 0.f;
+      }
+      i[u] = e + 32 * (U + u) < e1 ? F.pt_row[e + 32 * (U + u)] : -1;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < BF; ++q)
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[k] = fmaf(pv[u][q * K + k], rv[u][q], acc[k]);
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = warp_sum(acc[k]);
@@ -2336,9 +2395,89 @@ __device__ __forceinline__ void cyc_prolong(const CycLevel& F, const float* xc, 
   }
 }
 
+// The same onto level 0, a thread per block row: the row's columns and coarse
+// values are read once for its BF components (a thread per component read them
+// BF times), the next block's column ahead of the current block's values.
+template <int BF, int K>
+__device__ __forceinline__ void cyc_prolong_rows(const CycLevel& F, const float* xc, float* x, int64_t t0,
+                                                 int64_t stride) {
+  for (int64_t i = t0; i < F.n; i += stride) {
+    const int64_t e0 = F.p_ptr[i], e1 = F.p_ptr[i + 1];
+    if (e0 == e1) continue;
+    float s[BF], old[BF];
+#pragma unroll
+    for (int r = 0; r < BF; ++r) {
+      s[r] = 0.f;
+      old[r] = x[i * BF + r];
+    }
+    int c = F.p_col[e0];
+    for (int64_t e = e0; e < e1; ++e) {
+      float pv[BF * K], cv[K];
+      load_half<BF * K>(F.p_h + e * BF * K, pv);
+      load_row<K>(xc + (int64_t)c * K, cv);
+      if (e + 1 < e1) c = F.p_col[e + 1];
+#pragma unroll
+      for (int r = 0; r < BF; ++r)
+#pragma unroll
+        for (int k = 0; k < K; ++k) s[r] = fmaf(pv[r * K + k], cv[k], s[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < BF; ++r) x[i * BF + r] = old[r] + s[r];
+  }
+}
+
+// The pass of a scalar level on four rows by one warp, eight lanes to a row:
+// rows of ten to thirty values leave most of a warp idle and a warp with eight
+// rows to walk one after the other (1024 x 512 heat slab).
+template <int MODE>
+__device__ __forceinline__ void cyc_rows_scalar(const CycLevel& L, int64_t i0, int lane, uint64_t pol) {
+  constexpr int G = 8, U = 2;
+  const float* v = MODE == kOpS1 || MODE == kOpS4 ? L.d : MODE == kOpS2 ? L.db : L.x;  // of other CTAs too
+  const int sub = lane & (G - 1);
+  const int64_t i = i0 + lane / G;
+  float y = 0.f;
+  if (i < L.n) {
+    const int64_t e1 = L.a_ptr[i + 1];
+    for (int64_t e = L.a_ptr[i] + sub; e < e1; e += U * G) {
+      int c[U];
+      float m[U];
+#pragma unroll
+      for (int w = 0; w < U; ++w) {
+        c[w] = e + w * G < e1 ? ld_l2(L.a_col + e + w * G, pol) : -1;
+        m[w] = e + w * G < e1 ? ld_l2(L.a_val + e + w * G, pol) : 0.f;
+      }
+#pragma unroll
+      for (int w = 0; w < U; ++w) y = fmaf(m[w], c[w] >= 0 ? v[c[w]] : 0.f, y);
+    }
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o, G);
+  if (i < L.n && sub == 0) {
+    if constexpr (MODE == kOpS1) {
+      const float rn = L.f[i] - y, dn = L.c1 * L.d[i] + L.c2 * (L.dinv[i] * rn);
+      L.r[i] = rn;
+      L.db[i] = dn;
+      L.x[i] += dn;
+    } else if constexpr (MODE == kOpS2) {
+      L.r[i] -= y;
+    } else if constexpr (MODE == kOpS3) {
+      const float rn = L.f[i] - y, dn = L.theta_inv * (L.dinv[i] * rn);
+      L.r[i] = rn;
+      L.d[i] = dn;
+      L.xb[i] = L.x[i] + dn;
+    } else {
+      L.xb[i] += L.c1 * L.d[i] + L.c2 * (L.dinv[i] * (L.r[i] - y));
+    }
+  }
+}
+
 template <int K, int MODE>
 __device__ __forceinline__ void cyc_pass(const CycLevel& L, int lane, int64_t warp, int64_t n_warps, uint64_t pol) {
-  for (int64_t i = warp; i < L.n; i += n_warps) cyc_row<K, MODE>(L, i, lane, pol);
+  if constexpr (K == 1) {
+    for (int64_t i = warp * 4; i < L.n; i += n_warps * 4) cyc_rows_scalar<MODE>(L, i, lane, pol);
+  } else {
+    for (int64_t i = warp; i < L.n; i += n_warps) cyc_row<K, MODE>(L, i, lane, pol);
+  }
 }
 
 // The same pass on block row i by a whole CTA, for levels with fewer rows
@@ -2503,7 +2642,8 @@ __device__ __forceinline__ bool coarse_phases(const CycArgs& a, unsigned long lo
     if (!cyc_barrier(bar, c, next)) return false;
     const CycLevel& F = a.L[l];
     if (l == 0) {
-      cyc_prolong<B0, K>(F, a.L[1].xb, F.x, tid, n_threads);
+      if constexpr (B0 == 1) cyc_prolong<B0, K>(F, a.L[1].xb, F.x, tid, n_threads);
+      else cyc_prolong_rows<B0, K>(F, a.L[1].xb, F.x, tid, n_threads);
       break;
     }
     cyc_prolong<K, K>(F, a.L[l + 1].xb, F.x, tid, n_threads);
@@ -2516,7 +2656,7 @@ __device__ __forceinline__ bool coarse_phases(const CycArgs& a, unsigned long lo
 }
 
 template <int B0, int K>
-__global__ void __launch_bounds__(kCycT) k_coarse_cycle(CycArgs a) {
+__global__ void __launch_bounds__(kCycT, kCycPerSm) k_coarse_cycle(CycArgs a) {
   __shared__ float fs[kCoarseMaxDof];
   __shared__ float part[kCycT];
   if (amg_idle(a.ctrl)) return;
