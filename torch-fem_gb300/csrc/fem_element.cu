@@ -212,48 +212,68 @@ k_stiffness(const double* __restrict__ bt, const double* __restrict__ detj,
     for (int q = 0; q < ND; ++q) out[i * ND + q] = acc[i][q];
 }
 
-// FP64 element matrices of an isotropic material by moments, for the FP64
-// copy of the mixed solvers' sliced matrix.  For C = lambda I(x)I + 2 G Isym
-// the (a, b) block of Ke is
+// FP64 element matrices of an isotropic material by moments.  For
+// C = lambda I(x)I + 2 G Isym the (a, b) block of Ke is
 //   K_ab[i][k] = lambda M[i][k] + G M[k][i] + G tr(M) delta_ik,
 //   M = sum_ip w detJ t g_a g_b^T,
-// the same sum as k_stiffness's, regrouped.  A CTA takes iso_epb(NE)
-// elements: it stages their gradients g and the scaled gradients
-// w detJ t g of every integration point in shared memory once, then a thread
-// per (element, node pair a <= b) accumulates the 3x3 (2x2) moment and writes
-// K_ab and K_ba = K_ab^T.  NE (NE + 1) / 2 pairs of D^2 FMAs per point
-// instead of NE^2 rows of products: this GPU's FP64 pipe is narrow.
+// the same sum as k_stiffness's, regrouped.  A CTA takes iso_epb elements: it
+// stages their gradients g and the scaled gradients w detJ t g of every
+// integration point in shared memory once, then a thread per (element, node
+// pair a <= b) accumulates the 3x3 (2x2) moment and writes K_ab and
+// K_ba = K_ab^T.  NE (NE + 1) / 2 pairs of D^2 FMAs per point instead of NE^2
+// rows of products: this GPU's FP64 pipe is narrow, and bounds the kernel.  A
+// warp's FP64 instruction costs the same with idle lanes, so iso_epb fills whole
+// warps: eight 8-node hexahedra are nine warps (three were 3.4).  70^3
+// hexahedra: 2.0 ms, 2.9 with three elements, the point scale formed per
+// component and zeros added off the diagonal; k_stiffness 13.
 __host__ __device__ constexpr int iso_pairs(int ne) { return ne * (ne + 1) / 2; }
-__host__ __device__ constexpr int iso_epb(int ne) { return iso_pairs(ne) >= 128 ? 1 : 128 / iso_pairs(ne); }
+__host__ __device__ constexpr int iso_epb(int ne, int d, int nip) {
+  int best = 1, best_of = 0;  // occupied lanes in 1024
+  for (int k = 1; k * iso_pairs(ne) <= 320 && k * nip * (ne * d * 16 + 8) <= 40 * 1024; ++k) {
+    const int t = k * iso_pairs(ne), of = t * 1024 / ((t + 31) / 32 * 32);
+    if (best * iso_pairs(ne) < 96 || of > best_of) {
+      best = k;
+      best_of = of;
+    }
+  }
+  return best;
+}
 
 template <int NE, int D, int NIP>
-__global__ void __launch_bounds__(iso_epb(NE) * iso_pairs(NE))
+__global__ void __launch_bounds__(iso_epb(NE, D, NIP) * iso_pairs(NE))
 k_stiffness_iso64(const double* __restrict__ bt, const double* __restrict__ detj,
                   const double* __restrict__ weights, const double* __restrict__ thickness,
                   const double* __restrict__ mat, int64_t n_elem, double* __restrict__ ke) {
   constexpr int ND = NE * D;
   constexpr int NP = iso_pairs(NE);
-  constexpr int EPB = iso_epb(NE);
+  constexpr int EPB = iso_epb(NE, D, NIP);
   __shared__ double g_s[EPB][NIP][ND];   // g
   __shared__ double sg_s[EPB][NIP][ND];  // w detJ t g
+  __shared__ double sc_s[EPB][NIP];      // w detJ t
   const int64_t e0 = (int64_t)blockIdx.x * EPB;
-  for (int q = threadIdx.x; q < EPB * NIP * ND; q += blockDim.x) {
-    const int le = q / (NIP * ND);
-    const int ip = (q / ND) % NIP;
-    const int c = q % ND;
-    const int64_t e = e0 + le;
-    double g = 0.0, sc = 0.0;
-    if (e < n_elem) {
-      g = bt[((int64_t)ip * n_elem + e) * ND + c];
-      sc = weights[ip] * detj[(int64_t)ip * n_elem + e] * (thickness ? thickness[e] : 1.0);
-    }
-    g_s[le][ip][c] = g;
-    sg_s[le][ip][c] = sc * g;
-  }
-  __syncthreads();
   const int le = threadIdx.x / NP;
   const int64_t e = e0 + le;
-  if (le >= EPB || e >= n_elem) return;
+  const bool mine = le < EPB && e < n_elem;
+  const double lam = mine ? mat[e * 2] : 0.0, G = mine ? mat[e * 2 + 1] : 0.0;
+  for (int q = threadIdx.x; q < EPB * NIP; q += blockDim.x) {
+    const int64_t eq = e0 + q % EPB;
+    const int ip = q / EPB;
+    double sc = 0.0;
+    if (eq < n_elem) {
+      sc = weights[ip] * detj[(int64_t)ip * n_elem + eq];
+      if (thickness) sc *= thickness[eq];
+    }
+    sc_s[q % EPB][ip] = sc;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < EPB * NIP * ND; q += blockDim.x) {
+    const int ip = q / (EPB * ND), r = q % (EPB * ND), l = r / ND, c = r % ND;
+    const double g = e0 + l < n_elem ? bt[((int64_t)ip * n_elem + e0) * ND + r] : 0.0;
+    g_s[l][ip][c] = g;
+    sg_s[l][ip][c] = sc_s[l][ip] * g;
+  }
+  __syncthreads();
+  if (!mine) return;
   int p = threadIdx.x - le * NP;
   int a = 0;
   while (p >= NE - a) {  // pairs of row a: (a, a) .. (a, NE - 1)
@@ -279,7 +299,6 @@ k_stiffness_iso64(const double* __restrict__ bt, const double* __restrict__ detj
 #pragma unroll
       for (int k = 0; k < D; ++k) M[i][k] = fma(ga[i], gb[k], M[i][k]);
   }
-  const double lam = mat[e * 2], G = mat[e * 2 + 1];
   double tr = 0.0;
 #pragma unroll
   for (int i = 0; i < D; ++i) tr += M[i][i];
@@ -289,7 +308,8 @@ k_stiffness_iso64(const double* __restrict__ bt, const double* __restrict__ detj
   for (int i = 0; i < D; ++i)
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      const double v = lam * M[i][k] + G * M[k][i] + (i == k ? G * tr : 0.0);
+      double v = lam * M[i][k] + G * M[k][i];
+      if (i == k) v += G * tr;
       kab[i * ND + k] = v;
       kba[k * ND + i] = v;
     }
@@ -674,8 +694,9 @@ int fem_element_stiffness_iso64(const fem_mesh* m, const fem_material* mat, doub
   }
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                  \
-  k_stiffness_iso64<NE, D, NIP><<<(unsigned)((m->n_elem + iso_epb(NE) - 1) / iso_epb(NE)),          \
-                                  iso_epb(NE) * iso_pairs(NE), 0, st>>>(                           \
+  constexpr int kEpb = iso_epb(NE, D, NIP);                                                        \
+  k_stiffness_iso64<NE, D, NIP><<<(unsigned)((m->n_elem + kEpb - 1) / kEpb),                        \
+                                  kEpb * iso_pairs(NE), 0, st>>>(                                  \
       m->bt, m->detj, m->weights, m->thickness, mat->data, m->n_elem, ke);
       ::tfg::note_launch();
   TFG_DISPATCH_ETYPE(m->etype)
