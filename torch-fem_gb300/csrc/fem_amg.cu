@@ -1732,17 +1732,37 @@ void launch_sell(int64_t n, const int64_t* sell_base, const int32_t* sell_col, c
 }
 
 // The dot product of a level-0 pass that ends in one: the per-slice shares
-// left by k_sell_op added in a fixed order by one CTA, then the CG (or
-// Lanczos) scalar update.  Deterministic; idle exactly when the pass was.
+// left by the pass added in a fixed order by one cluster of kFinish CTAs, then
+// the CG (or Lanczos) scalar update.  Deterministic; idle exactly when the pass
+// was.  33,000 shares take one CTA of 1024 threads 15 us (33 loads a thread, then
+// 32 warps' FP64 additions on one SM's four pipes), the cluster 8; 11,200 shares
+// 12 us of one CTA.
+constexpr int kFinish = 8;
 template <int MODE>
-__global__ void __launch_bounds__(1024) k_dot_finish(int64_t n, OpArgs a) {
+__global__ void __cluster_dims__(kFinish, 1, 1) __launch_bounds__(256) k_dot_finish(int64_t n, OpArgs a) {
   __shared__ double red[32];
+  __shared__ double share[kFinish];
+  // every CTA has started before another writes to its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   pdl_enter();
-  if (amg_idle(a.ctrl)) return;
+  if (amg_idle(a.ctrl)) return;  // set again behind the next barrier only: the same in every CTA
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   double s = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(a.partial + i);
-  const double tot = block_sum(s, red);
-  if (threadIdx.x == 0) op_finish<MODE>(a, tot);
+#pragma unroll 4
+  for (int64_t i = rank * blockDim.x + threadIdx.x; i < n; i += kFinish * blockDim.x) s += __ldcg(a.partial + i);
+  s = block_sum_fixed(s, red);
+  if (threadIdx.x == 0) {
+    uint32_t to;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(amg_smem_u32(&share[rank])));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(s) : "memory");
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x < 32) {
+    const double tot = warp_sum_fixed(threadIdx.x < kFinish ? share[threadIdx.x] : 0.0);
+    if (threadIdx.x == 0) op_finish<MODE>(a, tot);
+  }
 }
 
 // The FP16 smoothing copy: max |a_ij| over the sliced FP32 values (as the
@@ -2774,10 +2794,12 @@ __global__ void __launch_bounds__(256) k_cg_update(int64_t n_nod, float* __restr
     }
     pre_step<D>(dinv, theta_inv, i, rv, d, mx);
   }
-  rr = block_sum(rr, red);
+  rr = block_sum_fixed(rr, red);
   if (threadIdx.x == 0) partial[blockIdx.x] = rr;
   if (arrive_last(&ctrl->counter)) {
-    const double t = sum_partials(partial, gridDim.x, 1, 0, red);
+    double t = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) t += __ldcg(partial + i);
+    t = block_sum_fixed(t, red);
     if (threadIdx.x == 0) {
       AmgCtrl* c = ctrl;
       c->counter = 0;
@@ -3713,7 +3735,7 @@ void launch_op(fem_amg* h, int l, const OpArgs& a, cudaStream_t st) {
     else
       launch_sell<B0, MODE, false>(L.n, h->sell_base, h->sell_col, h->sell_val, a, st);
     if constexpr (op_has_dot<MODE>()) {
-      launch_chain(1, 1024, 0, st, k_dot_finish<MODE>, ns, a);
+      launch_chain(kFinish, 256, 0, st, k_dot_finish<MODE>, ns, a);
       note_launch();
     }
     if (timed) cudaEventRecord(h->ev[2 * h->ev_used++ + 1], st);
@@ -3747,7 +3769,7 @@ int lanczos_level(fem_amg* h, int l, cudaStream_t st, double* rho) {
         const int64_t ns = (n + 31) / 32;
         launch_sell<B, kOpLzQ, false>(n, h->sell_base, h->sell_col, h->sell_val, a, st);
         note_launch();
-        k_dot_finish<kOpLzQ><<<1, 1024, 0, st>>>(ns, a);
+        k_dot_finish<kOpLzQ><<<kFinish, 256, 0, st>>>(ns, a);
         sliced = true;
       }
     }

@@ -56,6 +56,19 @@ static __device__ __noinline__ double2 warp_sum_fixed2(double a, double b) {
   return make_double2(v[0], v[1]);
 }
 
+// Block-level sum as block_sum, by warp_sum_fixed: FP64 additions in a tree
+// cost a warp 64 cycles of its sub-partition's pipe each.  Valid in warp 0.
+__device__ __forceinline__ double block_sum_fixed(double v, double* smem32) {
+  v = warp_sum_fixed(v);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) smem32[wid] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (wid == 0) t = warp_sum_fixed(lane < (int)(blockDim.x >> 5) ? smem32[lane] : 0.0);
+  __syncthreads();
+  return t;
+}
+
 // isfinite and == 0 by the bits: a comparison costs an FP64 instruction.
 __device__ __forceinline__ bool finite_bits(double v) { return ((__double2hiint(v) >> 20) & 0x7ff) != 0x7ff; }
 __device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
