@@ -1,0 +1,56 @@
+"""Conductivity matrices by node pairs at element counts around the elements a
+CTA takes, for every element type, with symmetric and unsymmetric kappa and a
+thickness, in FP64 and FP32, against einsum over the same gradients.
+
+An entry sums at most 8 x 3 products of five FP64 factors: relative error below
+40 x 2^-53 of the summed magnitudes, which exceed the largest entry by less than
+a factor of 20 on these meshes, so 1e-13 of that entry; FP32 entries are the FP64
+ones rounded (2^-24).
+"""
+
+import pytest
+import torch
+
+from torchfem_gb300 import PlanarHeat, SolidHeat, _lib, mesh
+from torchfem_gb300 import materials as M
+
+pytestmark = pytest.mark.gpu
+
+K3, K2 = M.IsotropicConductivity3D(1.0), M.IsotropicConductivity2D(1.0)
+HEXA, QUAD, TETRA = mesh.cube_hexa(4, 3, 6), mesh.rect_quad(8, 6), mesh.cube_tetra(3, 3, 3)
+TRIA = QUAD[0], torch.cat([QUAD[1][:, [0, 1, 2]], QUAD[1][:, [0, 2, 3]]])
+TYPES = {
+    "hexa1": (SolidHeat, HEXA, K3), "hexa2": (SolidHeat, mesh.linear_to_quadratic(*HEXA), K3),
+    "tetra1": (SolidHeat, TETRA, K3), "tetra2": (SolidHeat, mesh.linear_to_quadratic(*TETRA), K3),
+    "quad1": (PlanarHeat, QUAD, K2), "quad2": (PlanarHeat, mesh.linear_to_quadratic(*QUAD), K2),
+    "tria1": (PlanarHeat, TRIA, K2), "tria2": (PlanarHeat, mesh.linear_to_quadratic(*TRIA), K2),
+}
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 17, 25])
+@pytest.mark.parametrize("name", TYPES)
+def test_pairs_at_cta_remainders(cuda, name, n, symmetric):
+    model, (nodes, el), mat_ = TYPES[name]
+    gen = torch.Generator().manual_seed(n)
+    nodes = nodes + 0.02 * torch.rand(nodes.shape, generator=gen, dtype=torch.float64)
+    used, inv = torch.unique(el[:n], return_inverse=True)
+    m = model(nodes[used], inv.reshape(n, -1), mat_)
+    dm = m.device_mesh
+    _, mat, _refs = m._device_material()
+    d = nodes.shape[1]
+    kap = torch.eye(d, dtype=torch.float64) + 0.2 * torch.rand(n, d, d, generator=gen, dtype=torch.float64)
+    if symmetric:
+        kap = 0.5 * (kap + kap.transpose(1, 2))
+    kap = kap.to(cuda).contiguous()
+    th = 0.5 + torch.rand(n, generator=gen, dtype=torch.float64).to(cuda)
+    mesh_s, own = dm.make_mesh(th), _lib.FemMaterial(mat.kind, kap.data_ptr())
+    B = dm.bt.reshape(-1, n, el.shape[1], d)
+    w = dm.weights.to(cuda)[:, None] * dm.detj.reshape(-1, n) * th
+    ref = torch.einsum("pe,peai,eij,pebj->eab", w, B, kap, B)
+    k = dm.element_stiffness(mesh_s, own)
+    scale = float(ref.abs().max())
+    assert float((k - ref).abs().max()) <= 1e-13 * scale
+    assert not symmetric or torch.equal(k, k.transpose(1, 2))
+    k32 = dm.element_stiffness(mesh_s, own, torch.float32)
+    assert torch.equal(k32, k.float())

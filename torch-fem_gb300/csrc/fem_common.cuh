@@ -141,6 +141,23 @@ __device__ __forceinline__ double unit_scale(double norm2) {
     TFG_BODY;                             \
   } break;
 
+// Kernels with a thread per (element, node pair a <= b): the pairs of an element,
+// and the elements of a CTA, as many as fill whole warps best (a warp's FP64
+// instruction costs the same with idle lanes) within 320 threads and the shared
+// memory of two gradient tables.
+__host__ __device__ constexpr int node_pairs(int ne) { return ne * (ne + 1) / 2; }
+__host__ __device__ constexpr int pair_epb(int ne, int d, int nip) {
+  int best = 1, best_of = 0;  // occupied lanes in 1024
+  for (int k = 1; k * node_pairs(ne) <= 320 && k * nip * (ne * d * 16 + 8) <= 40 * 1024; ++k) {
+    const int t = k * node_pairs(ne), of = t * 1024 / ((t + 31) / 32 * 32);
+    if (best * node_pairs(ne) < 96 || of > best_of) {
+      best = k;
+      best_of = of;
+    }
+  }
+  return best;
+}
+
 #define TFG_DISPATCH_ETYPE(etype)                        \
   switch (etype) {                                       \
     TFG_ETYPE_CASE(FEM_QUAD1, 4, 2, 4)                   \

@@ -216,37 +216,24 @@ k_stiffness(const double* __restrict__ bt, const double* __restrict__ detj,
 // C = lambda I(x)I + 2 G Isym the (a, b) block of Ke is
 //   K_ab[i][k] = lambda M[i][k] + G M[k][i] + G tr(M) delta_ik,
 //   M = sum_ip w detJ t g_a g_b^T,
-// the same sum as k_stiffness's, regrouped.  A CTA takes iso_epb elements: it
+// the same sum as k_stiffness's, regrouped.  A CTA takes pair_epb elements: it
 // stages their gradients g and the scaled gradients w detJ t g of every
 // integration point in shared memory once, then a thread per (element, node
 // pair a <= b) accumulates the 3x3 (2x2) moment and writes K_ab and
 // K_ba = K_ab^T.  NE (NE + 1) / 2 pairs of D^2 FMAs per point instead of NE^2
 // rows of products: this GPU's FP64 pipe is narrow, and bounds the kernel.  A
-// warp's FP64 instruction costs the same with idle lanes, so iso_epb fills whole
+// warp's FP64 instruction costs the same with idle lanes, so pair_epb fills whole
 // warps: eight 8-node hexahedra are nine warps (three were 3.4).  70^3
 // hexahedra: 2.0 ms, 2.9 with three elements, the point scale formed per
 // component and zeros added off the diagonal; k_stiffness 13.
-__host__ __device__ constexpr int iso_pairs(int ne) { return ne * (ne + 1) / 2; }
-__host__ __device__ constexpr int iso_epb(int ne, int d, int nip) {
-  int best = 1, best_of = 0;  // occupied lanes in 1024
-  for (int k = 1; k * iso_pairs(ne) <= 320 && k * nip * (ne * d * 16 + 8) <= 40 * 1024; ++k) {
-    const int t = k * iso_pairs(ne), of = t * 1024 / ((t + 31) / 32 * 32);
-    if (best * iso_pairs(ne) < 96 || of > best_of) {
-      best = k;
-      best_of = of;
-    }
-  }
-  return best;
-}
-
 template <int NE, int D, int NIP>
-__global__ void __launch_bounds__(iso_epb(NE, D, NIP) * iso_pairs(NE))
+__global__ void __launch_bounds__(pair_epb(NE, D, NIP) * node_pairs(NE))
 k_stiffness_iso64(const double* __restrict__ bt, const double* __restrict__ detj,
                   const double* __restrict__ weights, const double* __restrict__ thickness,
                   const double* __restrict__ mat, int64_t n_elem, double* __restrict__ ke) {
   constexpr int ND = NE * D;
-  constexpr int NP = iso_pairs(NE);
-  constexpr int EPB = iso_epb(NE, D, NIP);
+  constexpr int NP = node_pairs(NE);
+  constexpr int EPB = pair_epb(NE, D, NIP);
   __shared__ double g_s[EPB][NIP][ND];   // g
   __shared__ double sg_s[EPB][NIP][ND];  // w detJ t g
   __shared__ double sc_s[EPB][NIP];      // w detJ t
@@ -694,9 +681,9 @@ int fem_element_stiffness_iso64(const fem_mesh* m, const fem_material* mat, doub
   }
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                  \
-  constexpr int kEpb = iso_epb(NE, D, NIP);                                                        \
+  constexpr int kEpb = pair_epb(NE, D, NIP);                                                        \
   k_stiffness_iso64<NE, D, NIP><<<(unsigned)((m->n_elem + kEpb - 1) / kEpb),                        \
-                                  kEpb * iso_pairs(NE), 0, st>>>(                                  \
+                                  kEpb * node_pairs(NE), 0, st>>>(                                  \
       m->bt, m->detj, m->weights, m->thickness, mat->data, m->n_elem, ke);
       ::tfg::note_launch();
   TFG_DISPATCH_ETYPE(m->etype)
