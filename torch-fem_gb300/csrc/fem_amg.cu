@@ -3289,6 +3289,8 @@ struct fem_amg {
   int32_t* status = nullptr;
   unsigned long long* counter = nullptr;
   std::vector<void*> mem;
+  char* block = nullptr;  // the current block: its unused part
+  size_t block_left = 0, block_sum = 0;
   int64_t dropped = 0;
   bool ready = false;
   // CUDA events around the level-0 SpMV launches of a chunk (timing on)
@@ -3317,12 +3319,38 @@ struct fem_amg {
   int cg_blocks = 0;
   unsigned long long* cg_sync = nullptr;
 
+  // Memory that lives as long as the handle.  A hierarchy takes some 140 pieces, most
+  // of them small, and a cudaMalloc costs 15 to 40 us and its cudaFree 10 to 30, so they
+  // are cut from blocks; a block doubles the sum of the earlier ones, from 2 up
+  // to 64 MB, and no more than the last is left unused.  Pieces of 16 MB and more are
+  // allocated by themselves.  Create and destroy of the hierarchy of 27 x 22 x 31
+  // hexahedra, wall time: 4.0 and 1.0 ms by single pieces, 3.3 and 0.4 from blocks.
   template <typename T>
   T* alloc(int64_t count, cudaStream_t st) {
-    void* p = nullptr;
-    const size_t bytes = (size_t)std::max<int64_t>(count, 1) * sizeof(T);
     (void)st;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
+    const size_t bytes = ((size_t)std::max<int64_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+    if (bytes > block_left) {
+      if (bytes >= ((size_t)16 << 20)) return alloc_own<T>(count);
+      const size_t size = std::max(bytes, std::min(std::max(block_sum, (size_t)2 << 20), (size_t)64 << 20));
+      char* b = alloc_own<char>((int64_t)size);
+      if (!b) {  // too little for a block: the piece alone
+        cudaGetLastError();
+        return alloc_own<T>(count);
+      }
+      block = b;
+      block_left = size;
+      block_sum += size;
+    }
+    T* p = reinterpret_cast<T*>(block);
+    block += bytes;
+    block_left -= bytes;
+    return p;
+  }
+  // Memory that may be given back before the handle goes.
+  template <typename T>
+  T* alloc_own(int64_t count) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, (size_t)std::max<int64_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
     mem.push_back(p);
     return static_cast<T*>(p);
   }
@@ -3822,7 +3850,7 @@ int setup_impl(fem_amg* h, const fem_matrix* A, cudaStream_t st) {
         h->dinv0_own = nullptr;
         h->dinv0_len = 0;
       }
-      h->dinv0_own = h->alloc<float>(len, st);
+      h->dinv0_own = h->alloc_own<float>(len);
       if (!h->dinv0_own) return check_cuda("AMG block-Jacobi copy");
       h->dinv0_len = len;
     }
@@ -3845,7 +3873,7 @@ int setup_impl(fem_amg* h, const fem_matrix* A, cudaStream_t st) {
         h->sv16 = nullptr;
         h->sv16_len = 0;
       }
-      h->sv16 = h->alloc<__half>(len, st);
+      h->sv16 = h->alloc_own<__half>(len);
       if (!h->sv16) return check_cuda("AMG FP16 smoothing copy");
       h->sv16_len = len;
     }
