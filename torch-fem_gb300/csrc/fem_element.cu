@@ -133,13 +133,14 @@ __device__ __forceinline__ const double* mat_ptr(int kind, const double* data, i
 }
 
 // --------------------------------------------------------------- stiffness --
-// Thread per (element, node a): accumulates the d x (n_e d) row block of a
-// over all integration points, then writes it contiguously.
+// Isotropic materials, general form.  Thread per (element, node a): accumulates
+// the d x (n_e d) row block of a over all integration points, then writes it
+// contiguously.
 template <int NE, int D, int NIP, typename T>
 __global__ void __launch_bounds__(128)
 k_stiffness(const double* __restrict__ bt, const double* __restrict__ detj,
             const double* __restrict__ weights, const double* __restrict__ thickness,
-            int kind, const double* __restrict__ mat, int64_t n_elem, T* __restrict__ ke) {
+            const double* __restrict__ mat, int64_t n_elem, T* __restrict__ ke) {
   constexpr int ND = NE * D;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_elem * NE) return;
@@ -157,52 +158,20 @@ k_stiffness(const double* __restrict__ bt, const double* __restrict__ detj,
     T ga[D];
 #pragma unroll
     for (int J = 0; J < D; ++J) ga[J] = (T)g[a * D + J];
-    const double* cmd = mat_ptr<D, NIP>(kind, mat, n_elem, e, ip);
-    if (kind == FEM_MAT_ISO) {
-      const T lam = (T)cmd[0] * s, G = (T)cmd[1] * s;
+    const T lam = (T)mat[e * 2] * s, G = (T)mat[e * 2 + 1] * s;
 #pragma unroll
-      for (int b = 0; b < NE; ++b) {
-        T gb[D];
+    for (int b = 0; b < NE; ++b) {
+      T gb[D];
 #pragma unroll
-        for (int J = 0; J < D; ++J) gb[J] = (T)g[b * D + J];
-        T dot = T(0);
+      for (int J = 0; J < D; ++J) gb[J] = (T)g[b * D + J];
+      T dot = T(0);
 #pragma unroll
-        for (int J = 0; J < D; ++J) dot += ga[J] * gb[J];
-#pragma unroll
-        for (int i = 0; i < D; ++i)
-#pragma unroll
-          for (int k = 0; k < D; ++k)
-            acc[i][b * D + k] += lam * ga[i] * gb[k] + G * ga[k] * gb[i] + (i == k ? G * dot : T(0));
-      }
-    } else {
-      // t[i][k][L] = sum_J ga[J] C[i][J][k][L]
-      T tt[D][D][D];
+      for (int J = 0; J < D; ++J) dot += ga[J] * gb[J];
 #pragma unroll
       for (int i = 0; i < D; ++i)
 #pragma unroll
         for (int k = 0; k < D; ++k)
-#pragma unroll
-          for (int L = 0; L < D; ++L) {
-            T v = T(0);
-#pragma unroll
-            for (int J = 0; J < D; ++J) v += ga[J] * (T)cmd[((i * D + J) * D + k) * D + L];
-            tt[i][k][L] = v * s;
-          }
-#pragma unroll
-      for (int b = 0; b < NE; ++b) {
-        T gb[D];
-#pragma unroll
-        for (int J = 0; J < D; ++J) gb[J] = (T)g[b * D + J];
-#pragma unroll
-        for (int i = 0; i < D; ++i)
-#pragma unroll
-          for (int k = 0; k < D; ++k) {
-            T v = T(0);
-#pragma unroll
-            for (int L = 0; L < D; ++L) v += tt[i][k][L] * gb[L];
-            acc[i][b * D + k] += v;
-          }
-      }
+          acc[i][b * D + k] += lam * ga[i] * gb[k] + G * ga[k] * gb[i] + (i == k ? G * dot : T(0));
     }
   }
   T* out = ke + (e * ND + (int64_t)a * D) * ND;
@@ -210,6 +179,84 @@ k_stiffness(const double* __restrict__ bt, const double* __restrict__ detj,
   for (int i = 0; i < D; ++i)
 #pragma unroll
     for (int q = 0; q < ND; ++q) out[i * ND + q] = acc[i][q];
+}
+
+// Element matrices for a tangent C per element or per integration point (not
+// symmetric in general).  A CTA takes tangent_epb elements; its threads first
+// form t[i][k][L] = w detJ t sum_J g_a[J] C[i][J][k][L] of every point and node a
+// in shared memory, a thread per (point, a, i), then a thread per node pair
+// accumulates K_ab[i][k] = sum t[i][k][L] g_b[L].  The FP64 pipe bounds a large
+// mesh, with the same operations as a thread per node row that keeps t to
+// itself; a small one is bounded by the length of a thread's chain, 1,500 FP64
+// instructions there for ten nodes and four points, 150 here.  By node rows and
+// here, us: 144 quadratic tetrahedra 76, 16; 256 quadrilaterals 14, 4.3; 97,336
+// hexahedra 4537, 3433 (FP32 1377, 1045); 160,000 quadrilaterals 368, 274.
+__host__ __device__ constexpr int tangent_epb(int ne, int d, int nip) {
+  int best = 1, best_of = 0;  // occupied lanes in 1024
+  for (int k = 1; k * ne * ne <= 320 && k * nip * ne * (d * d * d + d) * 8 <= 40 * 1024; ++k) {
+    const int t = k * ne * ne, of = t * 1024 / ((t + 31) / 32 * 32);
+    if (best * ne * ne < 96 || of > best_of) {
+      best = k;
+      best_of = of;
+    }
+  }
+  return best;
+}
+
+template <int NE, int D, int NIP, typename T>
+__global__ void __launch_bounds__(tangent_epb(NE, D, NIP) * NE * NE)
+k_stiffness_tangent(const double* __restrict__ bt, const double* __restrict__ detj,
+                    const double* __restrict__ weights, const double* __restrict__ thickness,
+                    int kind, const double* __restrict__ mat, int64_t n_elem, T* __restrict__ ke) {
+  constexpr int ND = NE * D, EPB = tangent_epb(NE, D, NIP), D3 = D * D * D;
+  __shared__ T g_s[EPB][NIP][ND];
+  __shared__ T t_s[EPB][NIP][NE][D3];
+  const int64_t e0 = (int64_t)blockIdx.x * EPB;
+  for (int q = threadIdx.x; q < EPB * NIP * ND; q += blockDim.x) {
+    const int i = q % D, a = q / D % NE, ip = q / ND % NIP, l = q / (ND * NIP);
+    const int64_t e = e0 + l, pe = (int64_t)ip * n_elem + e;
+    if (e >= n_elem) continue;
+    const T s = (T)weights[ip] * (T)detj[pe] * (thickness ? (T)thickness[e] : T(1));
+    const double* g = bt + (pe * NE + a) * D;
+    const double* c = mat_ptr<D, NIP>(kind, mat, n_elem, e, ip) + i * D3;
+    g_s[l][ip][a * D + i] = (T)g[i];
+    T ga[D];
+#pragma unroll
+    for (int J = 0; J < D; ++J) ga[J] = (T)g[J];
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+#pragma unroll
+      for (int L = 0; L < D; ++L) {
+        T v = T(0);
+#pragma unroll
+        for (int J = 0; J < D; ++J) v += ga[J] * (T)c[(J * D + k) * D + L];
+        t_s[l][ip][a][(i * D + k) * D + L] = v * s;
+      }
+  }
+  __syncthreads();
+  const int b = threadIdx.x % NE, a = threadIdx.x / NE % NE, l = threadIdx.x / (NE * NE);
+  const int64_t e = e0 + l;
+  if (e >= n_elem) return;
+  T acc[D][D];
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+#pragma unroll
+    for (int k = 0; k < D; ++k) acc[i][k] = T(0);
+  for (int ip = 0; ip < NIP; ++ip) {
+    T gb[D];
+#pragma unroll
+    for (int L = 0; L < D; ++L) gb[L] = g_s[l][ip][b * D + L];
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+      for (int k = 0; k < D; ++k)
+#pragma unroll
+        for (int L = 0; L < D; ++L) acc[i][k] += t_s[l][ip][a][(i * D + k) * D + L] * gb[L];
+  }
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+#pragma unroll
+    for (int k = 0; k < D; ++k) ke[(e * ND + a * D + i) * ND + b * D + k] = acc[i][k];
 }
 
 // FP64 element matrices of an isotropic material by moments.  For
@@ -703,16 +750,28 @@ int fem_element_stiffness(const fem_mesh* m, const fem_material* mat, int out_dt
   }
   if (out_dtype == FEM_F64) {
 #define TFG_BODY                                                                               \
-  k_stiffness<NE, D, NIP, double><<<grid_for(m->n_elem * NE, 128), 128, 0, st>>>(              \
-      m->bt, m->detj, m->weights, m->thickness, mat->kind, mat->data, m->n_elem, (double*)ke);
-      ::tfg::note_launch();
+  if (mat->kind == FEM_MAT_ISO) {                                                              \
+    k_stiffness<NE, D, NIP, double><<<grid_for(m->n_elem * NE, 128), 128, 0, st>>>(             \
+        m->bt, m->detj, m->weights, m->thickness, mat->data, m->n_elem, (double*)ke);           \
+  } else {                                                                                     \
+    constexpr int kEpb = tangent_epb(NE, D, NIP);                                              \
+    k_stiffness_tangent<NE, D, NIP, double><<<grid_for(m->n_elem, kEpb), kEpb * NE * NE, 0, st>>>( \
+        m->bt, m->detj, m->weights, m->thickness, mat->kind, mat->data, m->n_elem, (double*)ke); \
+  }                                                                                            \
+  ::tfg::note_launch();
     TFG_DISPATCH_ETYPE(m->etype)
 #undef TFG_BODY
   } else if (out_dtype == FEM_F32) {
 #define TFG_BODY                                                                               \
-  k_stiffness<NE, D, NIP, float><<<grid_for(m->n_elem * NE, 128), 128, 0, st>>>(               \
-      m->bt, m->detj, m->weights, m->thickness, mat->kind, mat->data, m->n_elem, (float*)ke);
-      ::tfg::note_launch();
+  if (mat->kind == FEM_MAT_ISO) {                                                              \
+    k_stiffness<NE, D, NIP, float><<<grid_for(m->n_elem * NE, 128), 128, 0, st>>>(             \
+        m->bt, m->detj, m->weights, m->thickness, mat->data, m->n_elem, (float*)ke);           \
+  } else {                                                                                     \
+    constexpr int kEpb = tangent_epb(NE, D, NIP);                                              \
+    k_stiffness_tangent<NE, D, NIP, float><<<grid_for(m->n_elem, kEpb), kEpb * NE * NE, 0, st>>>( \
+        m->bt, m->detj, m->weights, m->thickness, mat->kind, mat->data, m->n_elem, (float*)ke); \
+  }                                                                                            \
+  ::tfg::note_launch();
     TFG_DISPATCH_ETYPE(m->etype)
 #undef TFG_BODY
   } else {

@@ -56,9 +56,24 @@ __device__ __forceinline__ void inv3(const double (&F)[3][3], double J, double (
   Fi[2][2] = (F[0][0] * F[1][1] - F[0][1] * F[1][0]) * r;
 }
 
+// Threads of a CTA of the kernels with a thread per (element, point), and the
+// elements of such a CTA: as many as its threads hold, fewer where that leaves
+// SMs without any.
+constexpr int kPointT = 128;
+static int point_epb(int64_t n_elem, int nip) {
+  const int64_t spread = (n_elem + 151) / 152;
+  return (int)(spread < kPointT / nip ? spread : kPointT / nip);
+}
+
 // ------------------------------------------------------------ Neo-Hookean ---
 // P = mu F + (lambda ln J - mu) F^-T
 // A_iJkL = mu d_ik d_JL + lambda Fi_Ji Fi_Lk + (mu - lambda ln J) Fi_Jk Fi_Li
+// A thread per (element, integration point) for the point's state, then the
+// CTA's threads share out the tangent's rows and the nodal forces.  For a small
+// mesh the time is the FP64 instructions of one thread in a row (with a thread
+// per element: all its points, 81 tangent entries each), so point_epb also
+// spreads few elements over the SMs.  By elements and here, us: 144 quadratic
+// tetrahedra 76, 11; 1,728 hexahedra 166, 35; 97,336 hexahedra 714, 681.
 template <int NE, int NIP>
 __global__ void __launch_bounds__(128)
 k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
@@ -67,21 +82,16 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
         const uint8_t* __restrict__ con_mask, const double* __restrict__ con_values, int con_mode,
         const double* __restrict__ F_prev, double* __restrict__ fe, double* __restrict__ P_out,
         double* __restrict__ tangent, double* __restrict__ flux, double* __restrict__ F_out,
-        int32_t* status) {
+        int32_t* status, int epb) {
   constexpr int D = 3, ND = NE * D;
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n_elem) return;
-  double ve[NE][D];
-  load_field_nl<NE, D>(v, elements + e * NE, con_mask, con_values, con_mode, ve);
-  const double mu = params[e * 2 + 0], lam = params[e * 2 + 1];
-  double f[NE][D];
-#pragma unroll
-  for (int a = 0; a < NE; ++a)
-#pragma unroll
-    for (int c = 0; c < D; ++c) f[a][c] = 0.0;
-  bool ok = true;
-  for (int ip = 0; ip < NIP; ++ip) {
-    const int64_t pe = (int64_t)ip * n_elem + e;
+  __shared__ double P_s[kPointT][9], Fi_s[kPointT][9], c_s[kPointT][3];  // per point; mu, lambda, mu - lambda ln J
+  const int64_t e0 = (int64_t)blockIdx.x * epb;
+  const int le = threadIdx.x % epb, ip = threadIdx.x / epb;
+  const int64_t e = e0 + le, pe = (int64_t)ip * n_elem + e;
+  if (ip < NIP && e < n_elem) {
+    double ve[NE][D];
+    load_field_nl<NE, D>(v, elements + e * NE, con_mask, con_values, con_mode, ve);
+    const double mu = params[e * 2 + 0], lam = params[e * 2 + 1];
     const double* g = bt + pe * ND;
     double F[3][3];
 #pragma unroll
@@ -94,7 +104,7 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
         F[c][j] = s;
       }
     const double J = det3(F);
-    ok = ok && (J > 0.0);
+    if (!(J > 0.0)) flag_status(status, kStatNonFinite);
     double Fi[3][3];
     inv3(F, J, Fi);
     const double lnJ = log(J);
@@ -128,37 +138,57 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
         }
     }
     if (tangent) {
-      const double c2 = mu - lam * lnJ;
-      double* A = tangent + pe * 81;
+#pragma unroll
       for (int i = 0; i < 3; ++i)
-        for (int J2 = 0; J2 < 3; ++J2)
-          for (int k = 0; k < 3; ++k)
-            for (int L = 0; L < 3; ++L)
-              A[((i * 3 + J2) * 3 + k) * 3 + L] = (i == k && J2 == L ? mu : 0.0) + lam * Fi[J2][i] * Fi[L][k] +
-                                                  c2 * Fi[J2][k] * Fi[L][i];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) Fi_s[threadIdx.x][i * 3 + j] = Fi[i][j];
+      c_s[threadIdx.x][0] = mu;
+      c_s[threadIdx.x][1] = lam;
+      c_s[threadIdx.x][2] = mu - lam * lnJ;
     }
-    const double s = weights[ip] * detj[pe];
 #pragma unroll
-    for (int a = 0; a < NE; ++a)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int c = 0; c < D; ++c) {
-        double acc = 0.0;
-#pragma unroll
-        for (int j = 0; j < D; ++j) acc += g[a * D + j] * P[c][j];
-        f[a][c] += s * acc;
-      }
+      for (int j = 0; j < 3; ++j) P_s[threadIdx.x][i * 3 + j] = P[i][j];
   }
-  double* out = fe + e * ND;
+  __syncthreads();
+  if (tangent)
+    for (int q = threadIdx.x; q < epb * NIP * 9; q += kPointT) {  // a row (i, J2) of nine entries each
+      const int J2 = q % 3, i = q / 3 % 3, l = q / 9 % epb, p = q / (9 * epb);
+      const int64_t el = e0 + l;
+      if (el >= n_elem) continue;
+      const double* Fi = Fi_s[p * epb + l];
+      const double* c = c_s[p * epb + l];
+      double* A = tangent + ((int64_t)p * n_elem + el) * 81 + (i * 3 + J2) * 9;
+      const double lf = c[1] * Fi[J2 * 3 + i];
 #pragma unroll
-  for (int a = 0; a < NE; ++a)
+      for (int k = 0; k < 3; ++k) {
+        const double cf = c[2] * Fi[J2 * 3 + k];
 #pragma unroll
-    for (int c = 0; c < D; ++c) {
-      out[a * D + c] = f[a][c];
-      ok = ok && isfinite(f[a][c]);
+        for (int L = 0; L < 3; ++L)
+          A[k * 3 + L] = fma(cf, Fi[L * 3 + i], fma(lf, Fi[L * 3 + k], i == k && J2 == L ? c[0] : 0.0));
+      }
     }
-  if (!ok) flag_status(status, kStatNonFinite);
+  for (int q = threadIdx.x; q < epb * ND; q += kPointT) {
+    const int c = q % D, a = q / D % NE, l = q / ND;
+    const int64_t el = e0 + l;
+    if (el >= n_elem) break;
+    double f = 0.0;
+#pragma unroll
+    for (int p = 0; p < NIP; ++p) {
+      const double* g = bt + (((int64_t)p * n_elem + el) * NE + a) * D;
+      double acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < D; ++j) acc += g[j] * P_s[p * epb + l][c * 3 + j];
+      f += weights[p] * detj[(int64_t)p * n_elem + el] * acc;
+    }
+    fe[el * ND + a * D + c] = f;
+    if (!isfinite(f)) flag_status(status, kStatNonFinite);
+  }
 }
 
+// Reverse of k_hyper, threads likewise: 144 quadratic tetrahedra 131 us by
+// elements, 29 here; 97,336 hexahedra 815, 729.
 template <int NE, int NIP>
 __global__ void __launch_bounds__(128)
 k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
@@ -167,26 +197,22 @@ k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
             const uint8_t* __restrict__ con_mask, const double* __restrict__ con_values, int con_mode,
             const double* __restrict__ F_prev, const double* __restrict__ g_nodal,
             const double* __restrict__ gflux, const double* __restrict__ gF, double* __restrict__ gFprev,
-            double* __restrict__ gparams, double* __restrict__ gve) {
+            double* __restrict__ gparams, double* __restrict__ gve, int epb) {
   constexpr int D = 3, ND = NE * D;
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n_elem) return;
-  const int32_t* conn = elements + e * NE;
-  double ve[NE][D], ge[NE][D];
-  load_field_nl<NE, D>(v, conn, con_mask, con_values, con_mode, ve);
+  __shared__ double Fb_s[kPointT][9], gp_s[kPointT][2];
+  const int64_t e0 = (int64_t)blockIdx.x * epb;
+  const int le = threadIdx.x % epb, ip = threadIdx.x / epb;
+  const int64_t e = e0 + le, pe = (int64_t)ip * n_elem + e;
+  if (ip < NIP && e < n_elem) {
+    const int32_t* conn = elements + e * NE;
+    double ve[NE][D], ge[NE][D];
+    load_field_nl<NE, D>(v, conn, con_mask, con_values, con_mode, ve);
 #pragma unroll
-  for (int a = 0; a < NE; ++a)
+    for (int a = 0; a < NE; ++a)
 #pragma unroll
     for (int c = 0; c < D; ++c) ge[a][c] = g_nodal ? g_nodal[(int64_t)conn[a] * D + c] : 0.0;
-  const double mu = params[e * 2 + 0], lam = params[e * 2 + 1];
-  double gv[NE][D];
-#pragma unroll
-  for (int a = 0; a < NE; ++a)
-#pragma unroll
-    for (int c = 0; c < D; ++c) gv[a][c] = 0.0;
-  double gmu = 0.0, glam = 0.0;
-  for (int ip = 0; ip < NIP; ++ip) {
-    const int64_t pe = (int64_t)ip * n_elem + e;
+    const double mu = params[e * 2 + 0], lam = params[e * 2 + 1];
+    double gmu = 0.0, glam = 0.0;
     const double* g = bt + pe * ND;
     double F[3][3];
 #pragma unroll
@@ -286,25 +312,38 @@ k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
         for (int j = 0; j < 3; ++j) gFprev[pe * 9 + i * 3 + j] = Fb[i][j];
     }
 #pragma unroll
-    for (int a = 0; a < NE; ++a)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int c = 0; c < D; ++c) {
+      for (int j = 0; j < 3; ++j) Fb_s[threadIdx.x][i * 3 + j] = Fb[i][j];
+    gp_s[threadIdx.x][0] = gmu;
+    gp_s[threadIdx.x][1] = glam;
+  }
+  __syncthreads();
+  if (gparams)
+    for (int q = threadIdx.x; q < epb * 2; q += kPointT) {
+      const int64_t el = e0 + q / 2;
+      if (el >= n_elem) break;
+      double t = 0.0;
+#pragma unroll
+      for (int p = 0; p < NIP; ++p) t += gp_s[p * epb + q / 2][q % 2];
+      gparams[el * 2 + q % 2] = t;
+    }
+  if (gve)
+    for (int q = threadIdx.x; q < epb * ND; q += kPointT) {
+      const int c = q % D, a = q / D % NE, l = q / ND;
+      const int64_t el = e0 + l;
+      if (el >= n_elem) break;
+      double t = 0.0;
+#pragma unroll
+      for (int p = 0; p < NIP; ++p) {
+        const double* g = bt + (((int64_t)p * n_elem + el) * NE + a) * D;
         double acc = 0.0;
 #pragma unroll
-        for (int j = 0; j < D; ++j) acc += g[a * D + j] * Fb[c][j];
-        gv[a][c] += acc;
+        for (int j = 0; j < D; ++j) acc += g[j] * Fb_s[p * epb + l][c * 3 + j];
+        t += acc;
       }
-  }
-  if (gparams) {
-    gparams[e * 2 + 0] = gmu;
-    gparams[e * 2 + 1] = glam;
-  }
-  if (gve) {
-#pragma unroll
-    for (int a = 0; a < NE; ++a)
-#pragma unroll
-      for (int c = 0; c < D; ++c) gve[e * ND + a * D + c] = gv[a][c];
-  }
+      gve[el * ND + a * D + c] = t;
+    }
 }
 
 // ------------------------------------------------ J2 plasticity, plane strain
@@ -367,6 +406,8 @@ __device__ __forceinline__ void j2_update(double lam, double G, double E, double
   }
 }
 
+// Threads as in k_hyper.  By elements and here, us: 256 quadrilaterals 37, 11;
+// 40,000 quadratic ones 135, 121; 160,000 quadrilaterals 308, 320.
 template <int NE, int NIP>
 __global__ void __launch_bounds__(128)
 k_plastic(const double* __restrict__ bt, const double* __restrict__ detj,
@@ -376,23 +417,23 @@ k_plastic(const double* __restrict__ bt, const double* __restrict__ detj,
           const double* __restrict__ con_values, int con_mode, const double* __restrict__ sigma_prev,
           const double* __restrict__ state_prev, const double* __restrict__ de0, double* __restrict__ fe,
           double* __restrict__ sigma_out, double* __restrict__ state_out, double* __restrict__ tangent,
-          double* __restrict__ hgrad, int32_t* status) {
+          double* __restrict__ hgrad, int32_t* status, int epb) {
   constexpr int D = 2, ND = NE * D;
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n_elem) return;
-  double ve[NE][D];
-  load_field_nl<NE, D>(v, elements + e * NE, con_mask, con_values, con_mode, ve);
-  const double E = params[e * 4 + 0], nu = params[e * 4 + 1], sy = params[e * 4 + 2], Hh = params[e * 4 + 3];
-  const double lam = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), G = E / (2.0 * (1.0 + nu));
-  const double th = thickness ? thickness[e] : 1.0;
-  double f[NE][D];
-#pragma unroll
-  for (int a = 0; a < NE; ++a)
-#pragma unroll
-    for (int c = 0; c < D; ++c) f[a][c] = 0.0;
-  bool ok = true;
-  for (int ip = 0; ip < NIP; ++ip) {
-    const int64_t pe = (int64_t)ip * n_elem + e;
+  __shared__ double sig_s[kPointT][4], lame_s[kPointT][2];
+  const int64_t e0 = (int64_t)blockIdx.x * epb;
+  const int le = threadIdx.x % epb, ip = threadIdx.x / epb;
+  const int64_t e = e0 + le, pe = (int64_t)ip * n_elem + e;
+  if (ip == 0 && e < n_elem) {  // two divisions an element
+    const double E = params[e * 4 + 0], nu = params[e * 4 + 1];
+    lame_s[le][0] = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+    lame_s[le][1] = E / (2.0 * (1.0 + nu));
+  }
+  __syncthreads();
+  if (ip < NIP && e < n_elem) {
+    double ve[NE][D];
+    load_field_nl<NE, D>(v, elements + e * NE, con_mask, con_values, con_mode, ve);
+    const double E = params[e * 4 + 0], nu = params[e * 4 + 1], sy = params[e * 4 + 2], Hh = params[e * 4 + 3];
+    const double lam = lame_s[le][0], G = lame_s[le][1];
     const double* g = bt + pe * ND;
     double H[2][2];
 #pragma unroll
@@ -479,26 +520,29 @@ k_plastic(const double* __restrict__ bt, const double* __restrict__ detj,
           for (int k = 0; k < 2; ++k)
             for (int l = 0; l < 2; ++l) Tp[((i * 2 + j) * 2 + k) * 2 + l] = T[i][j][k][l];
     }
-    const double s = weights[ip] * detj[pe] * th;
 #pragma unroll
-    for (int a = 0; a < NE; ++a)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int c = 0; c < D; ++c) {
-        double acc = 0.0;
-#pragma unroll
-        for (int j = 0; j < D; ++j) acc += g[a * D + j] * sig[c][j];
-        f[a][c] += s * acc;
-      }
+      for (int j = 0; j < 2; ++j) sig_s[threadIdx.x][i * 2 + j] = sig[i][j];
   }
-  double* out = fe + e * ND;
+  __syncthreads();
+  for (int q = threadIdx.x; q < epb * ND; q += kPointT) {
+    const int c = q % D, a = q / D % NE, l = q / ND;
+    const int64_t el = e0 + l;
+    if (el >= n_elem) break;
+    const double th = thickness ? thickness[el] : 1.0;
+    double f = 0.0;
 #pragma unroll
-  for (int a = 0; a < NE; ++a)
+    for (int p = 0; p < NIP; ++p) {
+      const double* g = bt + (((int64_t)p * n_elem + el) * NE + a) * D;
+      double acc = 0.0;
 #pragma unroll
-    for (int c = 0; c < D; ++c) {
-      out[a * D + c] = f[a][c];
-      ok = ok && isfinite(f[a][c]);
+      for (int j = 0; j < D; ++j) acc += g[j] * sig_s[p * epb + l][c * 2 + j];
+      f += weights[p] * detj[(int64_t)p * n_elem + el] * th * acc;
     }
-  if (!ok) flag_status(status, kStatNonFinite);
+    fe[el * ND + a * D + c] = f;
+    if (!isfinite(f)) flag_status(status, kStatNonFinite);
+  }
 }
 
 // Reverse of k_plastic at the saved inputs (one increment's checkpoint).
@@ -714,9 +758,10 @@ int fem_hyper_force(const fem_mesh* m, const double* params, const double* v, co
   cudaStream_t st = as_stream(stream);
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                   \
-  k_hyper<NE, NIP><<<grid_for(m->n_elem, 128), 128, 0, st>>>(                                      \
+  const int epb = point_epb(m->n_elem, NIP);                                                        \
+  k_hyper<NE, NIP><<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                        \
       m->bt, m->detj, m->weights, m->elements, m->n_elem, params, v, con_mask, con_values, con_mode, \
-      F_prev, fe, P_out, tangent, flux, F_out, status);
+      F_prev, fe, P_out, tangent, flux, F_out, status, epb);
   TFG_NL3_DISPATCH(m->etype)
 #undef TFG_BODY
   ::tfg::note_launch();
@@ -730,9 +775,10 @@ int fem_hyper_vjp(const fem_mesh* m, const double* params, const double* v, cons
   cudaStream_t st = as_stream(stream);
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                    \
-  k_hyper_vjp<NE, NIP><<<grid_for(m->n_elem, 128), 128, 0, st>>>(                                   \
+  const int epb = point_epb(m->n_elem, NIP);                                                        \
+  k_hyper_vjp<NE, NIP><<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                        \
       m->bt, m->detj, m->weights, m->elements, m->n_elem, params, v, con_mask, con_values, con_mode, \
-      F_prev, g, gflux, gF, gFprev, gparams, gve);
+      F_prev, g, gflux, gF, gFprev, gparams, gve, epb);
   TFG_NL3_DISPATCH(m->etype)
 #undef TFG_BODY
   ::tfg::note_launch();
@@ -747,10 +793,11 @@ int fem_plastic_force(const fem_mesh* m, const double* params, double tol, int m
   cudaStream_t st = as_stream(stream);
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                    \
-  k_plastic<NE, NIP><<<grid_for(m->n_elem, 128), 128, 0, st>>>(                                     \
+  const int epb = point_epb(m->n_elem, NIP);                                                        \
+  k_plastic<NE, NIP><<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                        \
       m->bt, m->detj, m->weights, m->thickness, m->elements, m->n_elem, params, tol, max_iter, v,    \
       con_mask, con_values, con_mode, sigma_prev, state_prev, de0, fe, sigma_out, state_out, tangent, \
-      hgrad, status);
+      hgrad, status, epb);
   TFG_NL2_DISPATCH(m->etype)
 #undef TFG_BODY
   ::tfg::note_launch();
