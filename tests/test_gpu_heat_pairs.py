@@ -54,3 +54,37 @@ def test_pairs_at_cta_remainders(cuda, name, n, symmetric):
     assert not symmetric or torch.equal(k, k.transpose(1, 2))
     k32 = dm.element_stiffness(mesh_s, own, torch.float32)
     assert torch.equal(k32, k.float())
+
+
+WANTED = ["want_sig", "want_mat", "want_thick", "want_de0", "want_v"]
+
+
+@pytest.mark.parametrize("wants", [WANTED, [], *([w] for w in WANTED)])
+@pytest.mark.parametrize("name", ["hexa1", "tetra2", "quad1"])
+def test_reverse_of_fluxes(cuda, name, wants):
+    """Every output alone and all at once, against autograd over the formula
+    (the bound above; the reverse sums are as long)."""
+    model, (nodes, el), mat_ = TYPES[name]
+    gen = torch.Generator().manual_seed(4)
+    m = model(nodes, el, mat_)
+    dm, d, n = m.device_mesh, nodes.shape[1], len(el)
+    _, mat, _refs = m._device_material()
+    rnd = lambda *s: (torch.rand(s, generator=gen, dtype=torch.float64) - 0.3).to(cuda)  # noqa: E731
+    B, conn = dm.bt.reshape(-1, n, el.shape[1], d), el.to(cuda)
+    nip = B.shape[0]
+    leaves = rnd(nip, n, d), rnd(n, d, d), 1.0 + rnd(n), rnd(n, d), rnd(dm.n_dofs)
+    fp, kap, th, e0, v = (t.requires_grad_() for t in leaves)
+    g, gflux, gh = rnd(dm.n_dofs), rnd(nip, n, d), rnd(nip, n, d)
+    grad = torch.einsum("ea,peai->pei", v[conn], B)
+    flux = fp + torch.einsum("eij,pej->pei", kap, grad - e0)
+    w = dm.weights[:, None] * dm.detj.reshape(-1, n) * th
+    f = torch.einsum("pe,peai,pei->ea", w, B, flux)
+    refs = torch.autograd.grad((f * g[conn]).sum() + (flux * gflux).sum() + (grad * gh).sum(), (fp, kap, th, e0, v))
+    keep = [t.detach().contiguous() for t in leaves]
+    got = dm.vjp(dm.make_mesh(keep[2]), _lib.FemMaterial(mat.kind, keep[1].data_ptr()), keep[4], g,
+                 sigma_prev=keep[0], de0=keep[3], gflux=gflux, gh=gh, mat_numel=kap.numel(),
+                 **{k: True for k in wants})
+    for k, a, ref in zip(WANTED, got, refs):
+        assert (a is not None) == (k in wants)
+        if a is not None:
+            assert float((a.reshape(ref.shape) - ref).abs().max()) <= 1e-12 * float(ref.abs().max()), k
