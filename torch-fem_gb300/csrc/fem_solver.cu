@@ -1628,8 +1628,8 @@ __global__ void __launch_bounds__(128) k_csr_to_sell64(int64_t n_nod, int D, con
 }
 
 // ---------------------------------------------------- one-cluster FP64 CG ---
-// Small FP64 CSR systems.  A grid-wide persistent launch pays three grid
-// barriers and a chain of dependent L2 loads per iteration whatever the size.
+// Small FP64 CSR systems.  A grid-wide persistent launch pays two grid sums, a grid
+// barrier and a chain of dependent L2 loads per iteration whatever the size.
 // Here one thread-block cluster holds the whole system in its CTAs' shared
 // memory for the length of the solve: matrix values with 16-bit column codes
 // and, of the direction p, the window of columns that the CTA's rows touch.
@@ -1823,7 +1823,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
     lanes_s = best;
     fit_s = room && best >= 0;
     fail_s = 0;
-    if (best >= 0) info_s[2] = min(W, (R + (32 >> best) - 1) / (32 >> best));
+    if (best >= 0) info_s[2] = max(1, min(W, (R + (32 >> best) - 1) / (32 >> best)));
   }
   cl_sync();
   if (tid < 3 * (int)NC) all_s[tid / 3][tid % 3] = cl_ld(cl_map(smem_u32(&info_s[tid % 3]), tid / 3));
@@ -1849,10 +1849,11 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   uint16_t* row_s = code_s + (size_t)base_s[nb] * 32;  // rows by descending length
   for (int a = tid; a < R; a += T) row_s[a] = (uint16_t)perm_s[a];
   // where this CTA's shares go, and how many there are: the warps with blocks
-  // share p.q, the warps with rows r.z and r.r
+  // share p.q, the warps with rows r.z and r.r.  A CTA without rows sends one zero
+  // of each: nobody's next round then starts before it has read this one.
   int at_a = 0, at_b = 0, n_a = 0, n_b = 0;
   for (uint32_t c = 0; c < NC; ++c) {
-    const int wa = all_s[c][2], wb = min(W, (int)(lo_s[c + 1] - lo_s[c] + 31) / 32);
+    const int wa = all_s[c][2], wb = max(1, min(W, (int)(lo_s[c + 1] - lo_s[c] + 31) / 32));
     if (c < rank) {
       at_a += wa;
       at_b += wb;
@@ -1921,7 +1922,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   double total = 0.0;  // warp 0: r.z, warp 1: r.r
   auto reduce_rz_rr = [&](auto&& pre) {
     if (tid == 0) cl_expect(bar_b, 2 * n_b * (uint32_t)sizeof(double));
-    if (nu > 0) {
+    if (nu > 0 || warp == 0) {
       double2 s = make_double2(0.0, 0.0);
 #pragma unroll
       for (int u = 0; u < kClOwn; ++u) {
@@ -1974,7 +1975,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
         pq = fma(pw_s[own + row], s, pq);
       }
     }
-    if (warp < nb) {
+    if (warp < max(nb, 1)) {
       pq = warp_sum_fixed(pq);
       if (lane < (int)NC) cl_send(smem_u32(&part[0][at_a + warp]), bar_a, lane, pq);
     }
