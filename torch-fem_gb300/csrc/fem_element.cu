@@ -271,7 +271,7 @@ k_stiffness_tangent(const double* __restrict__ bt, const double* __restrict__ de
 // rows of products: this GPU's FP64 pipe is narrow, and bounds the kernel.  A
 // warp's FP64 instruction costs the same with idle lanes, so pair_epb fills whole
 // warps: eight 8-node hexahedra are nine warps (three were 3.4).  70^3
-// hexahedra: 2.0 ms, 2.9 with three elements, the point scale formed per
+// hexahedra: 2.1 ms, 2.9 with three elements, the point scale formed per
 // component and zeros added off the diagonal; k_stiffness 13.
 template <int NE, int D, int NIP>
 __global__ void __launch_bounds__(pair_epb(NE, D, NIP) * node_pairs(NE))

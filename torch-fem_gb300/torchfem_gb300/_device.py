@@ -349,7 +349,7 @@ class DeviceMesh:
 
     def element_stiffness64(self, mesh, mat) -> Tensor:
         """FP64 element matrices for a system of equations: the moment form
-        where the material is isotropic (70^3 hexahedra: 2.0 ms, 13 in the
+        where the material is isotropic (70^3 hexahedra: 2.1 ms, 13 in the
         general form), else the general form."""
         if not self.heat and mat.kind == _lib.FEM_MAT_ISO:
             return self.element_stiffness_iso64(mesh, mat)
