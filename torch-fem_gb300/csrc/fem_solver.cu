@@ -1729,8 +1729,14 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   __shared__ int base_s[kClBlocks + 1];          // first slot-row of every warp block
   __shared__ double part[3][kClMax * kClWarps];  // every warp's share of p.q, r.z and r.r
   __shared__ __align__(8) unsigned long long bar_s[3];
-  __shared__ double sh_scalar, sh_rz, sh_inv;
-  __shared__ int sh_done[2], fit_s, fail_s, lanes_s, cost_s[4], steps_s[4];
+  __shared__ double sh_rz, sh_inv;
+  // Decisions after r.z, after r.r and after p.q, and the two step lengths: a word each.
+  // A warp without rows or blocks sends no share, so the next sum completes without it
+  // and its total may be written while that warp still reads what the last one decided;
+  // of one word, a CTA barrier stands between its readers and its next writer.
+  __shared__ int sh_done[3];
+  __shared__ double sh_alpha, sh_beta;
+  __shared__ int fit_s, fail_s, lanes_s, cost_s[4], steps_s[4];
   __shared__ int info_s[3], all_s[kClMax][3];  // first and past-last column of the window, warps with blocks
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   constexpr int T = kClThreads, W = kClWarps;
@@ -1983,8 +1989,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
       if (!cl_wait(bar_a, phase_a)) fail_s = 1;
       const double v = cl_total(part[0], n_a);
       if (lane == 0) {
-        sh_scalar = rz / v;  // alpha
-        sh_done[0] = fail_s ? kDoneBarrierTimeout : !finite_bits(v) ? kDoneNonFinite : zero_bits(v) ? kDoneBreakdown
+        sh_alpha = rz / v;
+        sh_done[2] = fail_s ? kDoneBarrierTimeout : !finite_bits(v) ? kDoneNonFinite : zero_bits(v) ? kDoneBreakdown
                                                                                                     : kDoneNo;
       }
     } else if (tid == T - 1) {
@@ -1992,10 +1998,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
     }
     phase_a ^= 1;
     __syncthreads();
-    done = sh_done[0];
+    done = sh_done[2];
     if (done != kDoneNo) break;
     // ---- x += alpha p, r -= alpha q, z = M r
-    const double alpha = sh_scalar;
+    const double alpha = sh_alpha;
 #pragma unroll
     for (int u = 0; u < kClOwn; ++u) {
       if (u >= nu) break;
@@ -2013,7 +2019,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
     iters += 1;
     if (tid == 0) {
       sh_done[0] = fail_s ? kDoneBarrierTimeout : finite_bits(total) ? kDoneNo : kDoneNonFinite;
-      sh_scalar = total * sh_inv;  // beta
+      sh_beta = total * sh_inv;
       sh_rz = rz = total;
     }
     if (tid == 32)
@@ -2023,7 +2029,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
     __syncthreads();
     done = sh_done[0] ? sh_done[0] : sh_done[1];
     if (done != kDoneNo) break;
-    const double beta = sh_scalar;
+    const double beta = sh_beta;
 #pragma unroll
     for (int u = 0; u < kClOwn; ++u) {
       if (u >= nu) break;
