@@ -1665,6 +1665,8 @@ constexpr int kClSmem = 222 * 1024;  // dynamic shared memory per CTA
 constexpr int kClWide = 256;         // CTAs with more rows take one lane per row
 constexpr int kClBlocks = kClWide * 8 / 32;  // warp blocks of a CTA at most
 constexpr int kClNoFit = 100;        // ctrl->done: left to the grid-wide kernel
+constexpr int kClRowBytes = 2 * sizeof(double) + sizeof(uint16_t);  // shared memory of a row: p, q, its place
+constexpr int kClEntryBytes = sizeof(double) + sizeof(uint16_t);    // of a stored entry: value, column code
 
 struct ClusterParams {
   int64_t n;
@@ -1736,7 +1738,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   // of one word, a CTA barrier stands between its readers and its next writer.
   __shared__ int sh_done[3];
   __shared__ double sh_alpha, sh_beta;
-  __shared__ int fit_s, fail_s, lanes_s, cost_s[4], steps_s[4];
+  __shared__ int fit_s[2], fail_s, lanes_s, cost_s[4], steps_s[4];
   __shared__ int info_s[3], all_s[kClMax][3];  // first and past-last column of the window, warps with blocks
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   constexpr int T = kClThreads, W = kClWarps;
@@ -1756,9 +1758,22 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  // A system that is too large for some CTA is declined before its rows are
+  // ranked, which made a declined solve of two iterations 60 us longer (112 -> 175
+  // us, 16,384 rows): by its counts alone (p, q and a place per row, a value and a
+  // code per entry), every CTA from the same numbers, here (132 us), and by the
+  // window of columns, which only a CTA itself knows, below.
+  bool large = false;
+  if (tid < (int)NC) {
+    const int64_t rows = lo_s[tid + 1] - lo_s[tid], entries = P.row_ptr[lo_s[tid + 1]] - P.row_ptr[lo_s[tid]];
+    large = rows > kClRows || rows * kClRowBytes + entries * kClEntryBytes > kClSmem;
+  }
+  if (__syncthreads_or(large)) {
+    if (rank == 0 && tid == 0) P.ctrl->done = kClNoFit;
+    return;
+  }
   const int64_t row_lo = lo_s[rank];
-  const bool small = lo_s[rank + 1] - row_lo <= kClRows;
-  const int R = small ? (int)(lo_s[rank + 1] - row_lo) : 0;
+  const int R = (int)(lo_s[rank + 1] - row_lo);
   // the window of columns (n is at most kClMax * kClRows)
   if (tid == 0) {
     info_s[0] = (int)row_lo;
@@ -1789,13 +1804,24 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   int* len_s = reinterpret_cast<int*>(pw_s);  // set-up only: row lengths
   int* perm_s = reinterpret_cast<int*>(q_s);  // set-up only: rows by descending length
   const int fixed = (R + wn) * (int)sizeof(double) + R * (int)sizeof(uint16_t);
-  const int max_steps = (kClSmem - fixed) / (32 * 10);
-  const bool room = small && max_steps > 0;
-  const int Rs = room ? R : 0;  // rows of the set-up
-  for (int a = tid; a < Rs; a += T)
+  const int max_steps = (kClSmem - fixed) / (32 * kClEntryBytes);
+  // true in every CTA if every CTA holds true (flag k: of one vote)
+  auto vote = [&](int k) {
+    cl_sync();
+    int all = 1;
+    for (uint32_t c = 0; c < NC; ++c) all &= cl_ld(cl_map(smem_u32(&fit_s[k]), c));
+    return all != 0;
+  };
+  auto decline = [&] {
+    cl_sync();  // no CTA leaves while another reads its flag
+    if (rank == 0 && tid == 0) P.ctrl->done = kClNoFit;
+  };
+  if (tid == 0) fit_s[0] = fixed + (P.row_ptr[row_lo + R] - P.row_ptr[row_lo]) * kClEntryBytes <= kClSmem;
+  if (!vote(0)) return decline();
+  for (int a = tid; a < R; a += T)
     len_s[a] = (int)min((int64_t)(1 << 20), P.row_ptr[row_lo + a + 1] - P.row_ptr[row_lo + a]);
   __syncthreads();
-  for (int a = tid; a < Rs; a += T) {
+  for (int a = tid; a < R; a += T) {
     const int len = len_s[a];
     int place = 0;
     for (int i = 0; i < R; ++i) place += len_s[i] > len || (len_s[i] == len && i < a);
@@ -1808,8 +1834,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   if (tid < 4) {
     const int L = 1 << tid, rpb = 32 >> tid;
     int total = 0, steps = 0, longest = 0;
-    if (tid == 0 || Rs <= kClWide)
-      for (int k = 0; k * rpb < Rs && steps <= max_steps; ++k) {
+    if (tid == 0 || R <= kClWide)
+      for (int k = 0; k * rpb < R && steps <= max_steps; ++k) {
         const int st = (len_s[perm_s[k * rpb]] + L - 1) / L;
         const int ops = 2 * (st + 1) + 3 * tid;  // a shuffled addition costs half as much again
         steps += st;
@@ -1827,19 +1853,12 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
     for (int k = 0; k < 4; ++k)
       if (steps_s[k] <= max_steps && (best < 0 || cost_s[k] < cost_s[best])) best = k;
     lanes_s = best;
-    fit_s = room && best >= 0;
+    fit_s[1] = best >= 0;
     fail_s = 0;
     if (best >= 0) info_s[2] = max(1, min(W, (R + (32 >> best) - 1) / (32 >> best)));
   }
-  cl_sync();
+  if (!vote(1)) return decline();
   if (tid < 3 * (int)NC) all_s[tid / 3][tid % 3] = cl_ld(cl_map(smem_u32(&info_s[tid % 3]), tid / 3));
-  int fits = 1;
-  for (uint32_t c = 0; c < NC; ++c) fits &= cl_ld(cl_map(smem_u32(&fit_s), c));
-  if (!fits) {
-    cl_sync();  // no CTA leaves while another reads its flag
-    if (rank == 0 && tid == 0) P.ctrl->done = kClNoFit;
-    return;
-  }
   const int lsh = lanes_s, L = 1 << lsh, rpb = 32 >> lsh;
   const int nb = (R + rpb - 1) / rpb;
   if (tid == 0) {
