@@ -1,6 +1,7 @@
 """Which FP64 CSR systems the one-cluster CG takes, by the launches of a solve: one
 kernel there, a start and at least one more on the grid-wide path.  Edges: the
-rows of a cluster and its shared memory.  Both sides solve: the
+rows of a cluster, the shared memory, and the longest row (160 entries to a lane, one
+lane per row from 257 rows a CTA on, at most eight below).  Both sides solve: the
 matrices are A = diag(1 + row sums) + symmetric entries in [-1, 1], A >= I, so that
 ||b - A x|| <= rtol ||b|| up to the rounding of A x, below 2^-53 ||A||_1 ||x|| times
 the entries of a row, and ||A||_1 ||x|| <= 2 max(diag) ||b||.
@@ -47,6 +48,10 @@ CASES = {
     "most entries": (3900, list(range(1, 39)), 0, True),
     "too many entries": (4000, list(range(1, 50)), 0, False),
     "too wide a window": (16000, [1, 2, 3, 4, 8000, 15000], 0, False),
+    "single lanes, longest": (6000, WIDE, 160, True),
+    "single lanes, too long": (6000, WIDE, 161, False),
+    "eight lanes, longest": (1500, WIDE, 1280, True),
+    "eight lanes, too long": (1500, WIDE, 1281, False),
 }
 
 

@@ -1654,8 +1654,8 @@ __global__ void __launch_bounds__(128) k_csr_to_sell64(int64_t n_nod, int D, con
 // row on lane j % L): reads of the matrix are free of bank conflicts and little
 // padding is stored.  Every CTA sums the same shares in the same order, so
 // all take the same decisions and results are deterministic.  A system that
-// does not fit (shared memory, rows per CTA) is declined before the first
-// iteration and left to the grid-wide kernel.
+// does not fit (shared memory, rows per CTA) or has too long rows (kClLongest) is
+// declined before the first iteration and left to the grid-wide kernel.
 constexpr int kClMax = 16;        // CTAs per cluster (non-portable size; 8 where 16 cannot be placed)
 constexpr int kClThreads = 256;
 constexpr int kClWarps = kClThreads / 32;
@@ -1664,6 +1664,14 @@ constexpr int kClRows = kClOwn * kClThreads;
 constexpr int kClSmem = 222 * 1024;  // dynamic shared memory per CTA
 constexpr int kClWide = 256;         // CTAs with more rows take one lane per row
 constexpr int kClBlocks = kClWide * 8 / 32;  // warp blocks of a CTA at most
+// Steps of a block (its longest row's entries by the lanes of a row) at most.  The
+// warp of such a block walks them one after the other, about 50 ns each, however
+// little the others have to do; the grid-wide kernel gives a long row a whole CTA.
+// Rows of a point that drives a face, us an iteration, here / grid-wide: 4,500 rows
+// in single lanes, 100 steps 10.7 / 13.0, 200 15.6 / 15.2, 300 20.3 / 16.7, 400
+// 25.0 / 18.3; 2,500 rows in eight lanes, 113 steps 12.0 / 12.3, 175 14.8 / 12.9,
+// 275 19.0 / 13.0.
+constexpr int kClLongest = 160;
 constexpr int kClNoFit = 100;        // ctrl->done: left to the grid-wide kernel
 constexpr int kClRowBytes = 2 * sizeof(double) + sizeof(uint16_t);  // shared memory of a row: p, q, its place
 constexpr int kClEntryBytes = sizeof(double) + sizeof(uint16_t);    // of a stored entry: value, column code
@@ -1830,7 +1838,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   __syncthreads();
   // lanes per row: the fewest FP64 instructions in sequence (a block's steps,
   // its lane sums and its p.q product) on the busiest of four sub-partitions
-  // among those that fit; the longest row of a block is its first
+  // among those that fit and have no block too long; the longest row of a block is
+  // its first
   if (tid < 4) {
     const int L = 1 << tid, rpb = 32 >> tid;
     int total = 0, steps = 0, longest = 0;
@@ -1838,7 +1847,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
       for (int k = 0; k * rpb < R && steps <= max_steps; ++k) {
         const int st = (len_s[perm_s[k * rpb]] + L - 1) / L;
         const int ops = 2 * (st + 1) + 3 * tid;  // a shuffled addition costs half as much again
-        steps += st;
+        steps += st > kClLongest ? max_steps + 1 : st;
         total += ops;
         longest = max(longest, ops);
       }
