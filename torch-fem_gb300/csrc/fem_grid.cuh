@@ -89,12 +89,14 @@ __device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlo
 // the sum does not depend on the order of arrival.  The fixed point's scale
 // comes from the last sum of the same quantity, known to all: 2^-97 of it is
 // the unit, and a share up to 2^40 times as large fits.  A share beyond that
-// or not finite is marked in the words (nine bits above the count), and then,
-// like a first sum without a scale, the doubles themselves go round
-// (grid_sum_plain).  The words only ever grow and are read as differences; two
+// or not finite is marked in the words (nine bits above the count).  A sum below
+// 2^-35 of the last one has lost bits: every share was cut to the unit, 500 of them
+// by less than 2^-53 of a sum that large.  In either case, which every CTA sees in the
+// same words, and for a first sum without a scale, the doubles themselves go
+// round (grid_sum_plain).  The words only ever grow and are read as differences; two
 // sets alternate, since a CTA that adds to one again has seen every CTA in the
 // other, hence every CTA has read the first.
-constexpr int kSumWords = 4, kSumBits = 36;
+constexpr int kSumWords = 4, kSumBits = 36, kSumFall = 35;
 constexpr int kSumLine = 16;                                   // 8-byte words from one to the next
 constexpr int kSumHead = kSumLine * (1 + 2 * 2 * kSumWords);   // the counter, 2 sets of 2 values; plain slots follow
 struct GridSync {
@@ -229,13 +231,14 @@ __device__ __forceinline__ bool grid_sum(int* error, long long spin_limit, GridS
       }
       __syncwarp();
       good = __all_sync(0xffffffffu, good);
-      plain = __any_sync(0xffffffffu, ((delta >> 9) & 511) != 0);
       const long long sum = (long long)delta >> 18;
       double d = sum == 0 ? 0.0
                           : __longlong_as_double(__double_as_longlong((double)sum) +
                                                  ((long long)(kSumBits * word + ref - 1120) << 52));
       d += __shfl_xor_sync(0xffffffffu, d, 1);
       d += __shfl_xor_sync(0xffffffffu, d, 2);
+      const bool fell = ((__double2hiint(d) >> 20) & 0x7ff) < ref - kSumFall;
+      plain = __any_sync(0xffffffffu, part && (fell || ((delta >> 9) & 511) != 0));
 #pragma unroll
       for (int j = 0; j < NK; ++j) v[j] = __shfl_sync(0xffffffffu, d, j * kSumWords);
     }
