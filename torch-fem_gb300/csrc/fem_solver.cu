@@ -1985,7 +1985,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
   }
   if (tid == 32) {
     tol2 = P.rtol2 * bb;
-    sh_done[1] = !finite_bits(bb) ? kDoneNonFinite : (bb == 0.0 || bb <= tol2) ? kDoneConverged : kDoneNo;
+    sh_done[1] = fail_s ? kDoneBarrierTimeout
+                 : !finite_bits(bb) ? kDoneNonFinite : (bb == 0.0 || bb <= tol2) ? kDoneConverged : kDoneNo;
   }
   __syncthreads();
   int done = sh_done[0] ? sh_done[0] : sh_done[1];
@@ -2051,7 +2052,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(ClusterParams P) 
       sh_rz = rz = total;
     }
     if (tid == 32)
-      sh_done[1] = !finite_bits(total) ? kDoneNonFinite
+      sh_done[1] = fail_s ? kDoneBarrierTimeout
+                   : !finite_bits(total) ? kDoneNonFinite
                    : total <= tol2 ? kDoneConverged
                    : iters >= P.max_iter ? kDoneMaxIter : kDoneNo;
     __syncthreads();
