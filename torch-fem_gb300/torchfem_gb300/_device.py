@@ -264,7 +264,9 @@ class DeviceMesh:
         self._sell = None
 
     def sell(self):
-        """Sliced block layout of the node graph (built on first use)."""
+        """Sliced block layout of the node graph, built on first use: complete
+        before it is shown, since a solve in another thread may read it on
+        another stream."""
         if self._sell is None:
             L, st = self.lib, self.stream
             n_slices = (self.n_nod + 31) // 32
@@ -275,6 +277,7 @@ class DeviceMesh:
                   "fem_sell_layout")
             col = self._empty(max(n_slots.value, 1), torch.int32)
             check(L.fem_sell_columns(C.byref(self.blocks), ptr(base), ptr(col), st), "fem_sell_columns")
+            torch.cuda.current_stream(self.device).synchronize()
             self._sell = (base, col, n_slots.value)
         return self._sell
 
