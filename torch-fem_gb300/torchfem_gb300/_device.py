@@ -601,23 +601,30 @@ class DeviceMesh:
 
     def cg_matrix(self, sysm: LinearSystem) -> _lib.FemMatrix:
         """The matrix of an FP64 system as its CG reads it: the CSR form, or a
-        sliced block copy of the same values."""
+        sliced block copy of the same values where there is memory for one."""
         if sysm.cg_matrix is None:
             sysm.cg_matrix = sysm.matrix
             if self.d <= 3 and self.nnz > self.CG_CLUSTER_NNZ[self.d]:
-                base, col, n_slots = self.sell()
-                if n_slots * self.d * self.d <= self.CG_SELL_PAD * self.nnz:
-                    sysm.cg_val = self._empty(n_slots * self.d * self.d, torch.float64)
-                    check(
-                        self.lib.fem_csr_to_sell64(C.byref(self.blocks), ptr(self.row_ptr), ptr(sysm.val), ptr(base),
-                                                   ptr(sysm.cg_val), self.stream),
-                        "fem_csr_to_sell64",
-                    )
-                    sysm.cg_matrix = _lib.FemMatrix(
-                        _lib.FEM_FMT_SELL_F64, self.d, self.n_dofs, self.n_nod, ptr(base), ptr(col),
-                        ptr(sysm.cg_val), ptr(sysm.precond),
-                    )
+                try:
+                    self._sliced_copy(sysm)
+                except torch.OutOfMemoryError:
+                    pass  # the CSR form needs nothing more
         return sysm.cg_matrix
+
+    def _sliced_copy(self, sysm: LinearSystem) -> None:
+        base, col, n_slots = self.sell()
+        if n_slots * self.d * self.d > self.CG_SELL_PAD * self.nnz:
+            return
+        sysm.cg_val = self._empty(n_slots * self.d * self.d, torch.float64)
+        check(
+            self.lib.fem_csr_to_sell64(C.byref(self.blocks), ptr(self.row_ptr), ptr(sysm.val), ptr(base),
+                                       ptr(sysm.cg_val), self.stream),
+            "fem_csr_to_sell64",
+        )
+        sysm.cg_matrix = _lib.FemMatrix(
+            _lib.FEM_FMT_SELL_F64, self.d, self.n_dofs, self.n_nod, ptr(base), ptr(col), ptr(sysm.cg_val),
+            ptr(sysm.precond),
+        )
 
     def solve(self, sysm: LinearSystem, b: Tensor, rtol: float, max_iter: int | None = None,
               delta: float = 0.1, refine: bool = True, linear: str = "cg") -> Tensor:
