@@ -66,15 +66,6 @@ constexpr double kDropTol = 1e-10;  // relative pivot below which a mode is drop
 constexpr int kT = 256;             // threads of the row-parallel kernels
 constexpr int kSellW = 4;           // warps sharing one 32-row slice (level 0)
 
-int g_sm = 0;
-int sm_count() {
-  if (g_sm == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&g_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || g_sm <= 0) g_sm = 132;
-  }
-  return g_sm;
-}
 unsigned capped(int64_t blocks_needed, int per_sm) {
   const int64_t cap = (int64_t)sm_count() * per_sm;
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks_needed, cap));

@@ -28,6 +28,9 @@ void note_launch();
 // Converts a pending CUDA error into FEM_CUDA_ERROR with a message.
 int check_cuda(const char* where);
 
+// SM count of the current device (cached per host thread).
+int sm_count();
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline unsigned int grid_for(int64_t n, int threads) {

@@ -61,7 +61,7 @@ __device__ __forceinline__ void inv3(const double (&F)[3][3], double J, double (
 // SMs without any.
 constexpr int kPointT = 128;
 static int point_epb(int64_t n_elem, int nip) {
-  const int64_t spread = (n_elem + 151) / 152;
+  const int64_t spread = (n_elem + sm_count() - 1) / sm_count();
   return (int)(spread < kPointT / nip ? spread : kPointT / nip);
 }
 

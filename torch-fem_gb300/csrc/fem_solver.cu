@@ -2263,8 +2263,7 @@ __global__ void k_diag_barrier(Ctrl* c, unsigned long long* mem, long long spin_
 // ------------------------------------------------------------- host driver --
 constexpr int kThreads = 256;
 
-// SM count of the current device (cached per host thread).
-static int sm_count() {
+int sm_count() {
   static thread_local int n = 0;
   if (n == 0) {
     int dev = 0;
