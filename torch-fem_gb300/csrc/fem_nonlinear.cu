@@ -7,11 +7,10 @@
 //   J2 plasticity, plane strain, linear hardening sigma_f(q) = sigma_y + H q
 //     (IsotropicPlasticityPlaneStrain, materials/plasticity.py:430-590)
 //
-// Each kernel is one thread per element looping over its integration points:
-// it forms the increment gradient H from the nodal field, runs the material
-// update, accumulates the element forces f_e = sum w detJ t B^T P, and writes
-// the optional per-point outputs (stress, state, tangent, F).  The vjp
-// kernels recompute the point update from the saved inputs (the increment's
+// A point's thread (or an element's, point after point) forms the increment
+// gradient H from the nodal field, runs the material update and writes the
+// optional per-point outputs (stress, state, tangent, F); the element forces f_e =
+// sum w detJ t B^T P follow.  The vjp kernels recompute the point update from the saved inputs (the increment's
 // checkpoint) and pull cotangents back through it by hand.
 #include "fem_common.cuh"
 
@@ -63,6 +62,21 @@ constexpr int kPointT = 128;
 static int point_epb(int64_t n_elem, int nip) {
   const int64_t spread = (n_elem + sm_count() - 1) / sm_count();
   return (int)(spread < kPointT / nip ? spread : kPointT / nip);
+}
+
+// Whether a thread per element takes less time than one per (element, point).
+// Its time goes by waves of one CTA per SM, so with several points it does where the
+// waves are at least 4/5 full, as all large meshes' are.  us by elements / by points,
+// with tangent: plastic quadrilaterals 25,600 (1.3 waves) 71 / 59, 40,000 (2.06) 97 / 85,
+// 50,625 (2.6) 97 / 103, 75,625 (3.9) 129 / 148, 160,000 291 / 303, 640,000 1042 / 1193;
+// elastic ones 62,500 (3.2) 67 / 67, quadratic 62,500 91 / 96.  A single point leaves nothing to split but the nodal
+// sums, which pays while an SM has few elements: triangles, 4,050 7.7 / 6.8, 7,200 7.9 /
+// 7.3, 9,800 7.8 / 8.0, 20,000 11.8 / 14.1.
+constexpr int kSinglePoint = 64;  // elements per SM
+static bool plastic_by_elements(int64_t n_elem, int nip) {
+  if (nip == 1) return n_elem > (int64_t)kSinglePoint * sm_count();
+  const int64_t wave = (int64_t)kPointT * sm_count();
+  return (n_elem + wave - 1) / wave * wave * 4 <= n_elem * 5;
 }
 
 // ------------------------------------------------------------ Neo-Hookean ---
@@ -406,10 +420,12 @@ __device__ __forceinline__ void j2_update(double lam, double G, double E, double
   }
 }
 
-// Threads as in k_hyper.  By elements and here, us: 256 quadrilaterals 37, 11;
-// 40,000 quadratic ones 135, 121; 160,000 quadrilaterals 308, 320.
-template <int NE, int NIP>
-__global__ void __launch_bounds__(128)
+// Threads as in k_hyper, or (kElem) a thread per element, which keeps the nodal sums
+// in registers: no second pass over the gradients, no CTA barriers, one division
+// pair for all points.  Its time goes by whole waves of CTAs, so it serves the meshes
+// that fill them (plastic_by_elements).  The FP64 pipe bounds both.
+template <int NE, int NIP, bool kElem>
+__global__ void __launch_bounds__(kPointT)
 k_plastic(const double* __restrict__ bt, const double* __restrict__ detj,
           const double* __restrict__ weights, const double* __restrict__ thickness,
           const int32_t* __restrict__ elements, int64_t n_elem, const double* __restrict__ params,
@@ -419,21 +435,42 @@ k_plastic(const double* __restrict__ bt, const double* __restrict__ detj,
           double* __restrict__ sigma_out, double* __restrict__ state_out, double* __restrict__ tangent,
           double* __restrict__ hgrad, int32_t* status, int epb) {
   constexpr int D = 2, ND = NE * D;
-  __shared__ double sig_s[kPointT][4], lame_s[kPointT][2];
-  const int64_t e0 = (int64_t)blockIdx.x * epb;
-  const int le = threadIdx.x % epb, ip = threadIdx.x / epb;
-  const int64_t e = e0 + le, pe = (int64_t)ip * n_elem + e;
-  if (ip == 0 && e < n_elem) {  // two divisions an element
-    const double E = params[e * 4 + 0], nu = params[e * 4 + 1];
-    lame_s[le][0] = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
-    lame_s[le][1] = E / (2.0 * (1.0 + nu));
+  __shared__ double sig_s[kElem ? 1 : kPointT][4], lame_s[kElem ? 1 : kPointT][2];
+  const int64_t e0 = (int64_t)blockIdx.x * (kElem ? kPointT : epb);
+  const int le = kElem ? threadIdx.x : threadIdx.x % epb, ip0 = kElem ? 0 : threadIdx.x / epb;
+  const int64_t e = e0 + le;
+  const bool in = ip0 < NIP && e < n_elem;
+  double E = 0.0, nu = 0.0, lam = 0.0, G = 0.0;
+  if (in) {
+    E = params[e * 4 + 0];
+    nu = params[e * 4 + 1];
+    if (ip0 == 0) {  // two divisions an element
+      lam = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+      G = E / (2.0 * (1.0 + nu));
+    }
   }
-  __syncthreads();
-  if (ip < NIP && e < n_elem) {
-    double ve[NE][D];
-    load_field_nl<NE, D>(v, elements + e * NE, con_mask, con_values, con_mode, ve);
-    const double E = params[e * 4 + 0], nu = params[e * 4 + 1], sy = params[e * 4 + 2], Hh = params[e * 4 + 3];
-    const double lam = lame_s[le][0], G = lame_s[le][1];
+  if constexpr (!kElem) {
+    if (in && ip0 == 0) {
+      lame_s[le][0] = lam;
+      lame_s[le][1] = G;
+    }
+    __syncthreads();
+    if (in) {
+      lam = lame_s[le][0];
+      G = lame_s[le][1];
+    }
+  }
+  double ve[NE][D], f[kElem ? NE : 1][D];
+  if (in) load_field_nl<NE, D>(v, elements + e * NE, con_mask, con_values, con_mode, ve);
+  if constexpr (kElem) {
+#pragma unroll
+    for (int a = 0; a < NE; ++a)
+#pragma unroll
+      for (int c = 0; c < D; ++c) f[a][c] = 0.0;
+  }
+  for (int ip = ip0; in && ip < NIP; ip += kElem ? 1 : NIP) {
+    const int64_t pe = (int64_t)ip * n_elem + e;
+    const double sy = params[e * 4 + 2], Hh = params[e * 4 + 3];
     const double* g = bt + pe * ND;
     double H[2][2];
 #pragma unroll
@@ -520,10 +557,36 @@ k_plastic(const double* __restrict__ bt, const double* __restrict__ detj,
           for (int k = 0; k < 2; ++k)
             for (int l = 0; l < 2; ++l) Tp[((i * 2 + j) * 2 + k) * 2 + l] = T[i][j][k][l];
     }
+    if constexpr (kElem) {
+      const double s = weights[ip] * detj[pe] * (thickness ? thickness[e] : 1.0);
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int a = 0; a < NE; ++a)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) sig_s[threadIdx.x][i * 2 + j] = sig[i][j];
+        for (int c = 0; c < D; ++c) {
+          double acc = 0.0;
+#pragma unroll
+          for (int j = 0; j < D; ++j) acc += g[a * D + j] * sig[c][j];
+          f[a][c] += s * acc;
+        }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) sig_s[threadIdx.x][i * 2 + j] = sig[i][j];
+    }
+  }
+  if constexpr (kElem) {
+    bool ok = true;
+#pragma unroll
+    for (int a = 0; a < NE; ++a)
+#pragma unroll
+      for (int c = 0; c < D; ++c)
+        if (in) {
+          fe[e * ND + a * D + c] = f[a][c];
+          ok = ok && isfinite(f[a][c]);
+        }
+    if (!ok) flag_status(status, kStatNonFinite);
+    return;
   }
   __syncthreads();
   for (int q = threadIdx.x; q < epb * ND; q += kPointT) {
@@ -793,8 +856,10 @@ int fem_plastic_force(const fem_mesh* m, const double* params, double tol, int m
   cudaStream_t st = as_stream(stream);
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                    \
-  const int epb = point_epb(m->n_elem, NIP);                                                        \
-  k_plastic<NE, NIP><<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                        \
+  const bool elem = plastic_by_elements(m->n_elem, NIP);                                            \
+  const int epb = elem ? kPointT : point_epb(m->n_elem, NIP);                                       \
+  auto* kernel = elem ? k_plastic<NE, NIP, true> : k_plastic<NE, NIP, false>;                       \
+  kernel<<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                             \
       m->bt, m->detj, m->weights, m->thickness, m->elements, m->n_elem, params, tol, max_iter, v,    \
       con_mask, con_values, con_mode, sigma_prev, state_prev, de0, fe, sigma_out, state_out, tangent, \
       hgrad, status, epb);
