@@ -4,15 +4,17 @@ one, so that its results, checked elsewhere against autograd and the oracles, ar
 reference: its own form, on the same numbers.
 """
 
+import ctypes as C
+
 import pytest
 import torch
 
-from torchfem_gb300 import Planar, mesh
+from torchfem_gb300 import Planar, Solid, _lib, mesh
 from torchfem_gb300 import materials as M
 
 pytestmark = pytest.mark.gpu
 
-E2 = M.IsotropicElasticityPlaneStrain(1.0, 0.3)
+E3, E2 = M.IsotropicElasticity3D(1.0, 0.3), M.IsotropicElasticityPlaneStrain(1.0, 0.3)
 QUAD = mesh.rect_quad(5, 4)
 TRIA = QUAD[0], torch.cat([QUAD[1][:, [0, 1, 2]], QUAD[1][:, [0, 2, 3]]])
 PLANE = {"quad1": QUAD, "quad2": mesh.linear_to_quadratic(*QUAD), "tria1": TRIA,
@@ -76,3 +78,42 @@ def test_plastic_forms_agree(cuda, sms, name):
     for n in counts(per_sm * sms, 1.0) if name == "tria1" else counts(per_sm * sms, 4 / 5, 1.0, 2 * 4 / 5, 4.0):
         for got, want in zip(run(n), ref):
             assert close(got, want.repeat(1, -(-n // k), 1)[:, :n]), n
+
+
+def test_single_point_neo_hookean(cuda, sms):
+    """Linear tetrahedra: forces, tangents, fluxes and the reverse mode, some 200
+    roundings of numbers at most ten times the largest result: 1e-12 of it."""
+    gen = torch.Generator().manual_seed(6)
+    nodes, el = mesh.cube_tetra(3, 3, 3)
+    nodes = nodes + 0.02 * torch.rand(nodes.shape, generator=gen, dtype=torch.float64)
+    k = len(el)
+    rnd = lambda *s: torch.rand(s, generator=gen, dtype=torch.float64).to(cuda)  # noqa: E731
+    u, g = 0.002 * rnd(len(nodes), 3), rnd(len(nodes), 3) - 0.5
+    par, F0 = 0.5 + rnd(k, 2), torch.eye(3, dtype=torch.float64, device=cuda) + 0.05 * rnd(k, 3, 3)
+    gflux, gF = rnd(k, 3, 3) - 0.5, rnd(k, 3, 3) - 0.5
+
+    def run(n):
+        big, elements, c = copies(nodes, el, n)
+        m = Solid(big, elements, E3)
+        dm = m.device_mesh
+        ms, v, Fp, p = dm.make_mesh(None), u.repeat(c, 1).reshape(-1), tile(F0, n), tile(par, n)
+        out = dm.hyper_force(ms, p, v, F_prev=Fp, want_tangent=True, want_flux=True, want_F=True, want_P=True)
+        force = dm.hyper_force(ms, p, v, F_prev=Fp)[0]
+        dm.check_status("hyper")
+        assert close(force, out[0])
+        back = dm.hyper_vjp(ms, p, v, g.repeat(c, 1).reshape(-1), F_prev=Fp, gflux=tile(gflux, n), gF=tile(gF, n),
+                            want_Fprev=True, want_params=True)
+        return [t.reshape(n, -1) for t in (*out, *back[:2])] + [hyper_v(dm, ms, p, v, g, Fp, c, n)]
+
+    def hyper_v(dm, ms, p, v, g, Fp, c, n):
+        """The element sums of the nodal cotangents, before they meet at a node."""
+        gve = torch.full((n, 12), float("nan"), dtype=torch.float64, device=cuda)
+        gn = g.repeat(c, 1).reshape(-1).contiguous()
+        _lib.check(dm.lib.fem_hyper_vjp(C.byref(ms), p.data_ptr(), v.data_ptr(), None, None, 0, Fp.data_ptr(),
+                                        gn.data_ptr(), None, None, None, None, gve.data_ptr(), dm.stream), "vjp")
+        return gve
+
+    ref = run(k)
+    for n in counts(sms, 64, 512):
+        for got, want in zip(run(n), ref):
+            assert close(got, tile(want, n)), n

@@ -73,8 +73,12 @@ static int point_epb(int64_t n_elem, int nip) {
 // sums, which pays while an SM has few elements: triangles, 4,050 7.7 / 6.8, 7,200 7.9 /
 // 7.3, 9,800 7.8 / 8.0, 20,000 11.8 / 14.1.
 constexpr int kSinglePoint = 64;  // elements per SM
+constexpr int kOwnTangent = 512;
+static bool single_point(int64_t n_elem, int nip) {
+  return nip == 1 && n_elem > (int64_t)kSinglePoint * sm_count();
+}
 static bool plastic_by_elements(int64_t n_elem, int nip) {
-  if (nip == 1) return n_elem > (int64_t)kSinglePoint * sm_count();
+  if (nip == 1) return single_point(n_elem, nip);
   const int64_t wave = (int64_t)kPointT * sm_count();
   return (n_elem + wave - 1) / wave * wave * 4 <= n_elem * 5;
 }
@@ -88,17 +92,23 @@ static bool plastic_by_elements(int64_t n_elem, int nip) {
 // per element: all its points, 81 tangent entries each), so point_epb also
 // spreads few elements over the SMs.  By elements and here, us: 144 quadratic
 // tetrahedra 76, 11; 1,728 hexahedra 166, 35; 97,336 hexahedra 714, 681.
-template <int NE, int NIP>
-__global__ void __launch_bounds__(128)
+// kSingle (one point, meshes that give every SM elements enough): the thread sums
+// its element's forces itself, and writes its tangent too while the mesh is small
+// enough for that to hide (kOwnTangent).  Linear tetrahedra, us shared out / by the thread:
+// forces of 69,120 31.4 / 28.6, of 878,080 318 / 297; tangents of 16,875 19.3 / 17.5, of
+// 163,840 124 / 145.
+template <int NE, int NIP, bool kSingle>
+__global__ void __launch_bounds__(kPointT)
 k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
         const double* __restrict__ weights, const int32_t* __restrict__ elements, int64_t n_elem,
         const double* __restrict__ params, const double* __restrict__ v,
         const uint8_t* __restrict__ con_mask, const double* __restrict__ con_values, int con_mode,
         const double* __restrict__ F_prev, double* __restrict__ fe, double* __restrict__ P_out,
         double* __restrict__ tangent, double* __restrict__ flux, double* __restrict__ F_out,
-        int32_t* status, int epb) {
+        int32_t* status, int epb, bool own_tangent) {
   constexpr int D = 3, ND = NE * D;
-  __shared__ double P_s[kPointT][9], Fi_s[kPointT][9], c_s[kPointT][3];  // per point; mu, lambda, mu - lambda ln J
+  static_assert(!kSingle || NIP == 1, "one point");
+  __shared__ double P_s[kSingle ? 1 : kPointT][9], Fi_s[kPointT][9], c_s[kPointT][3];  // per point; mu, lambda, mu - lambda ln J
   const int64_t e0 = (int64_t)blockIdx.x * epb;
   const int le = threadIdx.x % epb, ip = threadIdx.x / epb;
   const int64_t e = e0 + le, pe = (int64_t)ip * n_elem + e;
@@ -151,7 +161,16 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
           flux[pe * 9 + i * 3 + j] = s / J;
         }
     }
-    if (tangent) {
+    if (kSingle && tangent && own_tangent) {
+      const double c2 = mu - lam * lnJ;
+      double* A = tangent + pe * 81;
+      for (int i = 0; i < 3; ++i)
+        for (int J2 = 0; J2 < 3; ++J2)
+          for (int k = 0; k < 3; ++k)
+            for (int L = 0; L < 3; ++L)
+              A[((i * 3 + J2) * 3 + k) * 3 + L] =
+                  fma(c2 * Fi[J2][k], Fi[L][i], fma(lam * Fi[J2][i], Fi[L][k], i == k && J2 == L ? mu : 0.0));
+    } else if (tangent) {
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -160,11 +179,28 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
       c_s[threadIdx.x][1] = lam;
       c_s[threadIdx.x][2] = mu - lam * lnJ;
     }
+    if constexpr (kSingle) {
+      const double s = weights[0] * detj[pe];
+      bool ok = true;
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+      for (int a = 0; a < NE; ++a)
 #pragma unroll
-      for (int j = 0; j < 3; ++j) P_s[threadIdx.x][i * 3 + j] = P[i][j];
+        for (int c = 0; c < D; ++c) {
+          double acc = 0.0;
+#pragma unroll
+          for (int j = 0; j < D; ++j) acc += g[a * D + j] * P[c][j];
+          fe[e * ND + a * D + c] = s * acc;
+          ok = ok && isfinite(s * acc);
+        }
+      if (!ok) flag_status(status, kStatNonFinite);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) P_s[threadIdx.x][i * 3 + j] = P[i][j];
+    }
   }
+  if (kSingle && (!tangent || own_tangent)) return;
   __syncthreads();
   if (tangent)
     for (int q = threadIdx.x; q < epb * NIP * 9; q += kPointT) {  // a row (i, J2) of nine entries each
@@ -183,6 +219,7 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
           A[k * 3 + L] = fma(cf, Fi[L * 3 + i], fma(lf, Fi[L * 3 + k], i == k && J2 == L ? c[0] : 0.0));
       }
     }
+  if constexpr (kSingle) return;
   for (int q = threadIdx.x; q < epb * ND; q += kPointT) {
     const int c = q % D, a = q / D % NE, l = q / ND;
     const int64_t el = e0 + l;
@@ -202,9 +239,10 @@ k_hyper(const double* __restrict__ bt, const double* __restrict__ detj,
 }
 
 // Reverse of k_hyper, threads likewise: 144 quadratic tetrahedra 131 us by
-// elements, 29 here; 97,336 hexahedra 815, 729.
-template <int NE, int NIP>
-__global__ void __launch_bounds__(128)
+// elements, 29 here; 97,336 hexahedra 815, 729; 878,080 linear tetrahedra 654 shared
+// out, 635 by the element's thread.
+template <int NE, int NIP, bool kSingle>
+__global__ void __launch_bounds__(kPointT)
 k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
             const double* __restrict__ weights, const int32_t* __restrict__ elements, int64_t n_elem,
             const double* __restrict__ params, const double* __restrict__ v,
@@ -213,7 +251,8 @@ k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
             const double* __restrict__ gflux, const double* __restrict__ gF, double* __restrict__ gFprev,
             double* __restrict__ gparams, double* __restrict__ gve, int epb) {
   constexpr int D = 3, ND = NE * D;
-  __shared__ double Fb_s[kPointT][9], gp_s[kPointT][2];
+  static_assert(!kSingle || NIP == 1, "one point");
+  __shared__ double Fb_s[kSingle ? 1 : kPointT][9], gp_s[kSingle ? 1 : kPointT][2];
   const int64_t e0 = (int64_t)blockIdx.x * epb;
   const int le = threadIdx.x % epb, ip = threadIdx.x / epb;
   const int64_t e = e0 + le, pe = (int64_t)ip * n_elem + e;
@@ -224,7 +263,7 @@ k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
 #pragma unroll
     for (int a = 0; a < NE; ++a)
 #pragma unroll
-    for (int c = 0; c < D; ++c) ge[a][c] = g_nodal ? g_nodal[(int64_t)conn[a] * D + c] : 0.0;
+      for (int c = 0; c < D; ++c) ge[a][c] = g_nodal ? g_nodal[(int64_t)conn[a] * D + c] : 0.0;
     const double mu = params[e * 2 + 0], lam = params[e * 2 + 1];
     double gmu = 0.0, glam = 0.0;
     const double* g = bt + pe * ND;
@@ -325,13 +364,32 @@ k_hyper_vjp(const double* __restrict__ bt, const double* __restrict__ detj,
 #pragma unroll
         for (int j = 0; j < 3; ++j) gFprev[pe * 9 + i * 3 + j] = Fb[i][j];
     }
+    if constexpr (kSingle) {
+      if (gparams) {
+        gparams[e * 2 + 0] = gmu;
+        gparams[e * 2 + 1] = glam;
+      }
+      if (gve) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+        for (int a = 0; a < NE; ++a)
 #pragma unroll
-      for (int j = 0; j < 3; ++j) Fb_s[threadIdx.x][i * 3 + j] = Fb[i][j];
-    gp_s[threadIdx.x][0] = gmu;
-    gp_s[threadIdx.x][1] = glam;
+          for (int c = 0; c < D; ++c) {
+            double acc = 0.0;
+#pragma unroll
+            for (int j = 0; j < D; ++j) acc += g[a * D + j] * Fb[c][j];
+            gve[e * ND + a * D + c] = acc;
+          }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) Fb_s[threadIdx.x][i * 3 + j] = Fb[i][j];
+      gp_s[threadIdx.x][0] = gmu;
+      gp_s[threadIdx.x][1] = glam;
+    }
   }
+  if constexpr (kSingle) return;
   __syncthreads();
   if (gparams)
     for (int q = threadIdx.x; q < epb * 2; q += kPointT) {
@@ -821,10 +879,13 @@ int fem_hyper_force(const fem_mesh* m, const double* params, const double* v, co
   cudaStream_t st = as_stream(stream);
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                   \
-  const int epb = point_epb(m->n_elem, NIP);                                                        \
-  k_hyper<NE, NIP><<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                        \
+  const bool single = single_point(m->n_elem, NIP);                                                \
+  const int epb = single ? kPointT : point_epb(m->n_elem, NIP);                                    \
+  auto* kernel = single ? k_hyper<NE, NIP, NIP == 1> : k_hyper<NE, NIP, false>;                    \
+  kernel<<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                            \
       m->bt, m->detj, m->weights, m->elements, m->n_elem, params, v, con_mask, con_values, con_mode, \
-      F_prev, fe, P_out, tangent, flux, F_out, status, epb);
+      F_prev, fe, P_out, tangent, flux, F_out, status, epb,                                        \
+      m->n_elem <= (int64_t)kOwnTangent * sm_count());
   TFG_NL3_DISPATCH(m->etype)
 #undef TFG_BODY
   ::tfg::note_launch();
@@ -838,8 +899,10 @@ int fem_hyper_vjp(const fem_mesh* m, const double* params, const double* v, cons
   cudaStream_t st = as_stream(stream);
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                    \
-  const int epb = point_epb(m->n_elem, NIP);                                                        \
-  k_hyper_vjp<NE, NIP><<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                        \
+  const bool single = single_point(m->n_elem, NIP);                                                 \
+  const int epb = single ? kPointT : point_epb(m->n_elem, NIP);                                     \
+  auto* kernel = single ? k_hyper_vjp<NE, NIP, NIP == 1> : k_hyper_vjp<NE, NIP, false>;             \
+  kernel<<<grid_for(m->n_elem, epb), kPointT, 0, st>>>(                                             \
       m->bt, m->detj, m->weights, m->elements, m->n_elem, params, v, con_mask, con_values, con_mode, \
       F_prev, g, gflux, gF, gFprev, gparams, gve, epb);
   TFG_NL3_DISPATCH(m->etype)
