@@ -117,3 +117,29 @@ def test_single_point_neo_hookean(cuda, sms):
     for n in counts(sms, 64, 512):
         for got, want in zip(run(n), ref):
             assert close(got, tile(want, n)), n
+
+
+@pytest.mark.parametrize("name", ["tetra1", "tria1"])
+def test_single_point_tangent_matrices(cuda, sms, name):
+    """FP64 and FP32 matrices of unsymmetric tangents, per element and per point: sums of
+    at most 9 products of a few factors, 40 x 2^-53 (2^-24) of the summed magnitudes, below
+    20 times the largest entry: 1e-13 and 1e-4 of it."""
+    gen = torch.Generator().manual_seed(7)
+    solid = name == "tetra1"
+    nodes, el = mesh.cube_tetra(3, 3, 3) if solid else TRIA
+    nodes = nodes + 0.02 * torch.rand(nodes.shape, generator=gen, dtype=torch.float64)
+    k, d = len(el), nodes.shape[1]
+    tangent = torch.rand(k, d**4, generator=gen, dtype=torch.float64).to(cuda)
+    th = 0.5 + torch.rand(k, generator=gen, dtype=torch.float64).to(cuda)
+
+    def run(n, kind, dtype):
+        big, elements, _ = copies(nodes, el, n)
+        dm = (Solid if solid else Planar)(big, elements, E3 if solid else E2).device_mesh
+        c, t = tile(tangent, n), tile(th, n)
+        return dm.element_stiffness(dm.make_mesh(t), _lib.FemMaterial(kind, c.data_ptr()), dtype)
+
+    for dtype, per_sm, tol in ((torch.float64, 192, 1e-13), (torch.float32, 1024, 1e-4)):
+        for kind in (_lib.FEM_MAT_GENERAL, _lib.FEM_MAT_TANGENT_IP):
+            ref = run(k, kind, dtype)
+            for n in counts(sms, per_sm):
+                assert close(run(n, kind, dtype), tile(ref, n), tol), n
