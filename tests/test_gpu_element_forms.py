@@ -9,7 +9,7 @@ import ctypes as C
 import pytest
 import torch
 
-from torchfem_gb300 import Planar, Solid, _lib, mesh
+from torchfem_gb300 import Planar, PlanarHeat, Solid, SolidHeat, _lib, mesh
 from torchfem_gb300 import materials as M
 
 pytestmark = pytest.mark.gpu
@@ -143,3 +143,30 @@ def test_single_point_tangent_matrices(cuda, sms, name):
             ref = run(k, kind, dtype)
             for n in counts(sms, per_sm):
                 assert close(run(n, kind, dtype), tile(ref, n), tol), n
+
+
+@pytest.mark.parametrize("name", ["hexa1", "tetra1", "tetra2", "quad1", "quad2", "tria1", "tria2"])
+def test_symmetric_conductivity_beside_another(cuda, name):
+    """An element's conductivity matrix is the same to the bit whatever its neighbours'
+    kappa, and symmetric where its own is."""
+    solid = name[:2] in ("he", "te")
+    grid = {"hexa": mesh.cube_hexa(4, 4, 6), "tetr": mesh.cube_tetra(3, 3, 4), "quad": QUAD, "tria": TRIA}[name[:4]]
+    nodes, el = mesh.linear_to_quadratic(*grid) if name[-1] == "2" else grid
+    gen = torch.Generator().manual_seed(8)
+    nodes = nodes + 0.02 * torch.rand(nodes.shape, generator=gen, dtype=torch.float64)
+    n, d = len(el), nodes.shape[1]
+    m = (SolidHeat if solid else PlanarHeat)(nodes, el, (M.IsotropicConductivity3D if solid else
+                                                         M.IsotropicConductivity2D)(1.0))
+    dm = m.device_mesh
+    _, mat, _refs = m._device_material()
+    kap = torch.eye(d, dtype=torch.float64) + 0.2 * torch.rand(n, d, d, generator=gen, dtype=torch.float64)
+    sym = (0.5 * (kap + kap.transpose(1, 2))).to(cuda).contiguous()
+    odd = torch.arange(n) % 7 == 3
+    mixed = torch.where(odd[:, None, None].to(cuda), kap.to(cuda), sym).contiguous()
+    k_sym, k_mixed = (dm.element_stiffness(dm.make_mesh(None), _lib.FemMaterial(mat.kind, k.data_ptr()))
+                      for k in (sym, mixed))
+    even = ~odd.to(cuda)
+    assert torch.equal(k_sym, k_sym.transpose(1, 2)) and torch.equal(k_sym[even], k_mixed[even])
+    B = dm.bt.reshape(-1, n, el.shape[1], d)
+    ref = torch.einsum("pe,peai,eij,pebj->eab", dm.weights[:, None] * dm.detj.reshape(-1, n), B, mixed, B)
+    assert close(k_mixed, ref, 1e-13)  # the bound of the conductivity tests

@@ -32,13 +32,31 @@ __device__ __forceinline__ void load_temps(const double* __restrict__ v, const i
   }
 }
 
+// kappa symmetric to the bit.
+template <int D>
+__device__ __forceinline__ bool same_as_transposed(const double (&kap)[D][D]) {
+  bool same = true;
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+#pragma unroll
+    for (int j = 0; j < i; ++j) same = same && __double_as_longlong(kap[i][j]) == __double_as_longlong(kap[j][i]);
+  return same;
+}
+
 // K_ab = sum_ip w detJ t B_a^T kappa B_b, bound by the narrow FP64 pipe.  A CTA
 // takes whole warps' worth of elements (pair_epb).  It stages the gradients B and
 // kappa^T B w detJ t of every integration point in shared memory, each formed
 // once; then a thread per (element, node pair a <= b) accumulates K_ab.  Where
-// kappa is symmetric to the bit K_ba is the same number; for other elements the
-// thread accumulates it as well.  524,288 hexahedra: 1.5 ms; with a thread per
-// node row, forming kappa^T B there and every pair twice, 2.7 ms.
+// kappa is symmetric to the bit K_ba is the same number; for other elements (a
+// rotated kappa may differ in its last bits) the thread accumulates it as well.
+// 524,288 hexahedra: 1.5 ms; with a thread per node row, forming kappa^T B there and
+// every pair twice, 2.7 ms.
+// One point (kVote) leaves a second sum no products to hide behind: if any
+// kappa of the CTA is unsymmetric, its threads take all pairs (a, b) in turn, a
+// symmetric element's lower half still from the same products.  878,080 linear
+// tetrahedra, us, symmetric / not: 138 / 165; with two sums a pair 132 / 176, by node
+// rows 163 / 163.  (More points lose more by the vote than that gains: hexahedra
+// 64,000 197 / 267 against 189 / 279.)
 template <int NE, int D, int NIP, typename T>
 __global__ void __launch_bounds__(pair_epb(NE, D, NIP) * node_pairs(NE))
 k_heat_stiffness(int64_t n_elem, const double* __restrict__ bt, const double* __restrict__ detj,
@@ -47,25 +65,55 @@ k_heat_stiffness(int64_t n_elem, const double* __restrict__ bt, const double* __
   constexpr int NP = node_pairs(NE), EPB = pair_epb(NE, D, NIP), ND = NE * D;
   __shared__ double b_s[EPB][NIP][ND];   // B
   __shared__ double kb_s[EPB][NIP][ND];  // w detJ t kappa^T B
+  constexpr bool kVote = NIP == 1;
+  __shared__ bool sym_s[kVote ? EPB : 1];
+  int other = 0;  // this thread has met an unsymmetric kappa
   const int64_t e0 = (int64_t)blockIdx.x * EPB;
   for (int q = threadIdx.x; q < EPB * NIP * NE; q += blockDim.x) {
     const int ip = q / (EPB * NE), l = q / NE % EPB, a = q % NE;
     const int64_t e = e0 + l, pe = (int64_t)ip * n_elem + e;
     if (e >= n_elem) continue;
     const double wj = w[ip] * detj[pe] * (thick ? thick[e] : 1.0);
-    double g[D];
+    double g[D], kap[D][D];
 #pragma unroll
     for (int i = 0; i < D; ++i) g[i] = bt[(pe * NE + a) * D + i];
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+      for (int j = 0; j < D; ++j) kap[i][j] = kappa[(e * D + i) * D + j];
 #pragma unroll
     for (int j = 0; j < D; ++j) {
       double s = 0.0;
 #pragma unroll
-      for (int i = 0; i < D; ++i) s += g[i] * kappa[(e * D + i) * D + j];
+      for (int i = 0; i < D; ++i) s += g[i] * kap[i][j];
       b_s[l][ip][a * D + j] = g[j];
       kb_s[l][ip][a * D + j] = s * wj;
     }
+    if constexpr (kVote) {
+      const bool symmetric = same_as_transposed<D>(kap);
+      if (a == 0) sym_s[l] = symmetric;
+      other |= !symmetric;
+    }
   }
-  __syncthreads();
+  auto entry = [&](int l, int a, int b) {
+    double s = 0.0;
+#pragma unroll
+    for (int ip = 0; ip < NIP; ++ip)
+#pragma unroll
+      for (int j = 0; j < D; ++j) s = fma(kb_s[l][ip][a * D + j], b_s[l][ip][b * D + j], s);
+    return s;
+  };
+  if constexpr (kVote) other = __syncthreads_or(other);
+  else __syncthreads();
+  if (kVote && other) {
+    for (int q = threadIdx.x; q < EPB * NE * NE; q += blockDim.x) {
+      const int b = q % NE, a = q / NE % NE, l = q / (NE * NE);
+      if (e0 + l >= n_elem) break;
+      const bool swap = a > b && sym_s[l];
+      ke[((e0 + l) * NE + a) * NE + b] = (T)entry(l, swap ? b : a, swap ? a : b);
+    }
+    return;
+  }
   const int le = threadIdx.x / NP;
   const int64_t e = e0 + le;
   if (le >= EPB || e >= n_elem) return;
@@ -76,28 +124,73 @@ k_heat_stiffness(int64_t n_elem, const double* __restrict__ bt, const double* __
     ++a;
   }
   const int b = a + p;
-  bool symmetric = true;
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-#pragma unroll
-    for (int j = 0; j < i; ++j)
-      symmetric = symmetric && __double_as_longlong(kappa[(e * D + i) * D + j]) ==
-                                   __double_as_longlong(kappa[(e * D + j) * D + i]);
-  double s = 0.0;
-#pragma unroll
-  for (int ip = 0; ip < NIP; ++ip)
-#pragma unroll
-    for (int j = 0; j < D; ++j) s = fma(kb_s[le][ip][a * D + j], b_s[le][ip][b * D + j], s);
+  const double s = entry(le, a, b);
   double t = s;
-  if (!symmetric && a != b) {
-    t = 0.0;
+  if constexpr (!kVote) {
+    bool symmetric = true;
 #pragma unroll
-    for (int ip = 0; ip < NIP; ++ip)
+    for (int i = 0; i < D; ++i)
 #pragma unroll
-      for (int j = 0; j < D; ++j) t = fma(kb_s[le][ip][b * D + j], b_s[le][ip][a * D + j], t);
+      for (int j = 0; j < i; ++j)
+        symmetric = symmetric && __double_as_longlong(kappa[(e * D + i) * D + j]) ==
+                                     __double_as_longlong(kappa[(e * D + j) * D + i]);
+    if (!symmetric && a != b) t = entry(le, b, a);
   }
   ke[(e * NE + a) * NE + b] = (T)s;
   ke[(e * NE + b) * NE + a] = (T)t;
+}
+
+// The same for one-point triangles, a thread per (element, node row): three nodes
+// and one point are too little for two stages around a barrier, memory latency
+// bounds the pair form.  A symmetric element's row writes its entries right of the
+// diagonal to both of their places.  us by pairs / by rows: 12,800 triangles 3.7 /
+// 3.1, 320,000 35.5 / 26.6, 1,280,000 135 / 100.
+template <int NE, int D, typename T>
+__global__ void __launch_bounds__(128)
+k_heat_stiffness_one(int64_t n_elem, const double* __restrict__ bt, const double* __restrict__ detj,
+                     const double* __restrict__ w, const double* __restrict__ kappa,
+                     const double* __restrict__ thick, T* __restrict__ ke) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n_elem * NE) return;
+  const int64_t e = t / NE;
+  const int a = (int)(t % NE);
+  const double wj = w[0] * detj[e] * (thick ? thick[e] : 1.0);
+  const double* B = bt + e * NE * D;
+  double kap[D][D], kb[D];
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+#pragma unroll
+    for (int j = 0; j < D; ++j) kap[i][j] = kappa[(e * D + i) * D + j];
+  const bool symmetric = same_as_transposed<D>(kap);
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < D; ++i) s += B[a * D + i] * kap[i][j];
+    kb[j] = s * wj;
+  }
+  T* k = ke + e * NE * NE;
+#pragma unroll
+  for (int b = 0; b < NE; ++b) {
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < D; ++j) s = fma(kb[j], B[b * D + j], s);
+    const T v = (T)s;
+    if (b >= a || !symmetric) k[a * NE + b] = v;
+    if (b > a && symmetric) k[b * NE + a] = v;
+  }
+}
+
+template <int NE, int D, int NIP, typename T>
+static void launch_heat_stiffness(const fem_mesh* m, const double* kappa, T* ke, cudaStream_t st) {
+  if constexpr (NIP == 1 && NE == 3) {
+    k_heat_stiffness_one<NE, D, T><<<grid_for(m->n_elem * NE, 128), 128, 0, st>>>(
+        m->n_elem, m->bt, m->detj, m->weights, kappa, m->thickness, ke);
+  } else {
+    constexpr int kEpb = pair_epb(NE, D, NIP);
+    k_heat_stiffness<NE, D, NIP, T><<<grid_for(m->n_elem, kEpb), kEpb * node_pairs(NE), 0, st>>>(
+        m->n_elem, m->bt, m->detj, m->weights, kappa, m->thickness, ke);
+  }
 }
 
 // Thread per element: gradient increment g = B v, flux = flux_prev +
@@ -284,7 +377,7 @@ __global__ void k_heat_mass(int64_t n_elem, const double* __restrict__ detj, con
   const int64_t e = t / NE;
   const int a = (int)(t % NE);
   const double c = rho[e] * (thick ? thick[e] : 1.0);
-  double row[NE];
+  double row[NE] = {};
 #pragma unroll
   for (int b = 0; b < NE; ++b) row[b] = 0.0;
   for (int ip = 0; ip < NIP; ++ip) {
@@ -386,17 +479,11 @@ int fem_heat_stiffness(const fem_mesh* m, const double* kappa, int out_dtype, vo
   if (rc) return rc;
   cudaStream_t st = as_stream(stream);
 #define TFG_BODY                                                                                         \
-  {                                                                                                      \
-    constexpr int kEpb = pair_epb(NE, D, NIP), kT = kEpb * node_pairs(NE);                               \
-    const unsigned g = grid_for(m->n_elem, kEpb);                                                        \
-    if (out_dtype == FEM_F32)                                                                            \
-      k_heat_stiffness<NE, D, NIP, float><<<g, kT, 0, st>>>(m->n_elem, m->bt, m->detj, m->weights, kappa, \
-                                                            m->thickness, static_cast<float*>(ke));      \
-    else                                                                                                 \
-      k_heat_stiffness<NE, D, NIP, double><<<g, kT, 0, st>>>(m->n_elem, m->bt, m->detj, m->weights, kappa, \
-                                                             m->thickness, static_cast<double*>(ke));    \
-    ::tfg::note_launch();                                                                                \
-  }
+  if (out_dtype == FEM_F32)                                                              \
+    launch_heat_stiffness<NE, D, NIP>(m, kappa, static_cast<float*>(ke), st);            \
+  else                                                                                   \
+    launch_heat_stiffness<NE, D, NIP>(m, kappa, static_cast<double*>(ke), st);           \
+  ::tfg::note_launch();
   TFG_DISPATCH_ETYPE(m->etype)
 #undef TFG_BODY
   return check_cuda("fem_heat_stiffness");
