@@ -170,3 +170,29 @@ def test_symmetric_conductivity_beside_another(cuda, name):
     B = dm.bt.reshape(-1, n, el.shape[1], d)
     ref = torch.einsum("pe,peai,eij,pebj->eab", dm.weights[:, None] * dm.detj.reshape(-1, n), B, mixed, B)
     assert close(k_mixed, ref, 1e-13)  # the bound of the conductivity tests
+
+
+@pytest.mark.parametrize("name", ["hexa1", "tetra1", "tetra2", "quad2", "tria1"])
+def test_moment_form_of_few_and_many(cuda, sms, name):
+    """Isotropic FP64 matrices where small CTAs end: the same sums, so the same to the
+    bit, and against the general form within its bound."""
+    solid = name[:2] in ("he", "te")
+    nodes, el = {"hexa1": mesh.cube_hexa(4, 3, 3), "tetra1": mesh.cube_tetra(3, 3, 2),
+                 "tetra2": mesh.linear_to_quadratic(*mesh.cube_tetra(2, 3, 2)),
+                 "quad2": mesh.linear_to_quadratic(*QUAD), "tria1": TRIA}[name]
+    nodes = nodes + 0.02 * torch.rand(nodes.shape, generator=torch.Generator().manual_seed(9), dtype=torch.float64)
+    k = len(el)
+    E = 1.0 + torch.arange(k, dtype=torch.float64) / k
+
+    def run(n):
+        big, elements, _ = copies(nodes, el, n)
+        mat = (M.IsotropicElasticity3D if solid else M.IsotropicElasticityPlaneStrain)(tile(E, n), torch.tensor(0.3))
+        m = (Solid if solid else Planar)(big, elements, mat)
+        mesh_s, mat, _refs = m._device_material()
+        dm = m.device_mesh
+        return dm.element_stiffness_iso64(mesh_s, mat), dm.element_stiffness(mesh_s, mat)
+
+    ref, general = run(k)
+    assert close(ref, general, 1e-13)
+    for n in counts(sms, 64 if name in ("tetra1", "tria1") else 4):
+        assert torch.equal(run(n)[0], tile(ref, n)), n

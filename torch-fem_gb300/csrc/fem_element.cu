@@ -342,15 +342,23 @@ static void launch_tangent(const fem_mesh* m, const fem_material* mat, T* ke, cu
 // warp's FP64 instruction costs the same with idle lanes, so pair_epb fills whole
 // warps: eight 8-node hexahedra are nine warps (three were 3.4).  70^3
 // hexahedra: 2.1 ms, 2.9 with three elements, the point scale formed per
-// component and zeros added off the diagonal; k_stiffness 13.
-template <int NE, int D, int NIP>
-__global__ void __launch_bounds__(pair_epb(NE, D, NIP) * node_pairs(NE))
+// component and zeros added off the diagonal; k_stiffness 13.  On few elements the
+// time is that of one CTA: smaller ones then (iso_few), of one element where that is
+// a warp of pairs at least, of 64 threads for one-point elements.  us with pair_epb
+// / so: 64 hexahedra 11.8 / 6.7, 512 11.9 / 10.1, 1,000 12.1 / 15.2; quadratic tetrahedra
+// 135 7.3 / 5.2, 320 7.5 / 6.5, 1,080 11.2 / 12.2; quadratic quadrilaterals 576 5.2 / 4.9,
+// 1,600 7.8 / 8.4; linear tetrahedra 135 5.0 / 3.9, 3,645 7.9 / 7.3, 8,640 12.0 / 11.8.
+__host__ __device__ constexpr int iso_few(int ne, int d, int nip) {
+  return node_pairs(ne) >= 32 ? 1 : nip == 1 ? 64 / node_pairs(ne) : pair_epb(ne, d, nip);
+}
+constexpr int iso_few_per_sm(int nip) { return nip == 1 ? 64 : 4; }  // elements
+template <int NE, int D, int NIP, int EPB>
+__global__ void __launch_bounds__(EPB * node_pairs(NE))
 k_stiffness_iso64(const double* __restrict__ bt, const double* __restrict__ detj,
                   const double* __restrict__ weights, const double* __restrict__ thickness,
                   const double* __restrict__ mat, int64_t n_elem, double* __restrict__ ke) {
   constexpr int ND = NE * D;
   constexpr int NP = node_pairs(NE);
-  constexpr int EPB = pair_epb(NE, D, NIP);
   __shared__ double g_s[EPB][NIP][ND];   // g
   __shared__ double sg_s[EPB][NIP][ND];  // w detJ t g
   __shared__ double sc_s[EPB][NIP];      // w detJ t
@@ -798,10 +806,11 @@ int fem_element_stiffness_iso64(const fem_mesh* m, const fem_material* mat, doub
   }
   if (m->n_elem == 0) return FEM_OK;
 #define TFG_BODY                                                                                  \
-  constexpr int kEpb = pair_epb(NE, D, NIP);                                                        \
-  k_stiffness_iso64<NE, D, NIP><<<(unsigned)((m->n_elem + kEpb - 1) / kEpb),                        \
-                                  kEpb * node_pairs(NE), 0, st>>>(                                  \
-      m->bt, m->detj, m->weights, m->thickness, mat->data, m->n_elem, ke);
+  constexpr int kEpb = pair_epb(NE, D, NIP), kFew = iso_few(NE, D, NIP);                            \
+  const int epb = m->n_elem <= (int64_t)iso_few_per_sm(NIP) * sm_count() ? kFew : kEpb;             \
+  auto* kernel = epb == kFew ? k_stiffness_iso64<NE, D, NIP, kFew> : k_stiffness_iso64<NE, D, NIP, kEpb>; \
+  kernel<<<grid_for(m->n_elem, epb), epb * node_pairs(NE), 0, st>>>(                                \
+      m->bt, m->detj, m->weights, m->thickness, mat->data, m->n_elem, ke);                          \
       ::tfg::note_launch();
   TFG_DISPATCH_ETYPE(m->etype)
 #undef TFG_BODY
