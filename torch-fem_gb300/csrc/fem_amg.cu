@@ -3332,8 +3332,9 @@ struct fem_amg {
   // fused coarse cycle: CTAs (0 not yet sized, -1 unavailable) and barrier state
   int cyc_blocks = 0;
   tfg::CycBarrier* cyc_bar = nullptr;
-  // fused CG: CTAs (0 not yet sized, -1 unavailable) and its grid_sum memory
-  int cg_blocks = 0;
+  // fused CG: CTAs with the FP32 and with the FP16 smoother (0 not yet sized, -1
+  // unavailable on this device) and its grid_sum memory
+  int cg_blocks[2] = {0, 0};
   unsigned long long* cg_sync = nullptr;
 
   // Memory that lives as long as the handle.  A hierarchy takes some 140 pieces, most
@@ -4096,7 +4097,8 @@ void launch_iteration(fem_amg* h, cudaStream_t st) {
 }
 
 // CG iterations as one launch of k_amg_cg, until they stop.  Returns false where
-// the system is too large for it to pay or the launch is refused.  By the bytes
+// the system is too large for it to pay or the launch is refused (a device shared
+// with other work may not hold the grid now and do so later).  By the bytes
 // of a smoothing pass (FP16 values and columns): up to 16 MB one CTA per SM, with
 // registers to load a row's epilogue before its product, then two; beyond 64 MB
 // the bulk copies of the separate launches stream the matrix faster.  Measured
@@ -4109,30 +4111,31 @@ constexpr int64_t kFusedOne = 16 << 20, kFusedMost = 64 << 20;
 template <int B0, int K>
 bool launch_fused_cg(fem_amg* h, cudaStream_t st) {
   const int64_t slots = h->sv16_len / (B0 * B0), pass = slots * (2 * B0 * B0 + 4);
-  if (h->cg_blocks < 0 || pass > kFusedMost) return false;
   const bool half = h->sv16 && g_amg_half;
+  int& blocks = h->cg_blocks[half];
+  if (blocks < 0 || pass > kFusedMost) return false;
   const bool one = pass <= kFusedOne;
   const void* kernel = half ? (one ? (const void*)k_amg_cg<B0, K, true, 1> : (const void*)k_amg_cg<B0, K, true, 2>)
                             : (one ? (const void*)k_amg_cg<B0, K, false, 1> : (const void*)k_amg_cg<B0, K, false, 2>);
-  if (h->cg_blocks == 0) {
+  if (blocks == 0) {
     int dev = 0, coop = 0, occ = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kCycT, 0) != cudaSuccess || occ < 1) {
       cudaGetLastError();
-      h->cg_blocks = -1;
+      blocks = -1;
+      return false;
+    }
+    const int most = std::min(kCycPerSm * sm_count(), 500);
+    if (!h->cg_sync)
+      h->cg_sync = h->alloc<unsigned long long>((int64_t)(sync_bytes(most) / sizeof(unsigned long long)), st);
+    if (!h->cg_sync) {
+      cudaGetLastError();
       return false;
     }
     // a group of warps per slice, as far as the GPU holds them
     const int64_t ns = (h->L[0].n + 31) / 32, per = kCycT / 32 / (B0 > 1 ? kSellW : 1);
-    h->cg_blocks = (int)std::max<int64_t>(
-        1, std::min<int64_t>((ns + per - 1) / per, std::min(std::min(occ, kCycPerSm) * sm_count(), 500)));
-    h->cg_sync = h->alloc<unsigned long long>((int64_t)(sync_bytes(h->cg_blocks) / sizeof(unsigned long long)), st);
-    if (!h->cg_sync) {
-      cudaGetLastError();
-      h->cg_blocks = -1;
-      return false;
-    }
+    blocks = (int)std::max<int64_t>(1, std::min<int64_t>((ns + per - 1) / per, std::min(occ * sm_count(), most)));
   }
   FusedArgs fa;
   fa.cyc = cycle_args(h);
@@ -4146,12 +4149,11 @@ bool launch_fused_cg(fem_amg* h, cudaStream_t st) {
   fa.xlo = h->xlo;
   fa.r = h->rcg;
   fa.sync = h->cg_sync;
-  cudaMemsetAsync(h->cg_sync, 0, sync_bytes(h->cg_blocks), st);
+  cudaMemsetAsync(h->cg_sync, 0, sync_bytes(blocks), st);
   cudaMemsetAsync(h->cyc_bar, 0, sizeof(CycBarrier), st);
   void* args[] = {&fa};
-  if (cudaLaunchCooperativeKernel(kernel, dim3(h->cg_blocks), dim3(kCycT), args, 0, st) != cudaSuccess) {
+  if (cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kCycT), args, 0, st) != cudaSuccess) {
     cudaGetLastError();
-    h->cg_blocks = -1;
     return false;
   }
   note_launch();
@@ -4225,6 +4227,7 @@ int pcg_impl(fem_amg* h, const fem_matrix* A, const fem_operator64* op, const do
     h->ev_ready = true;
   }
   const bool timing = g_timing && h->ev_ready;
+  bool fused = !timing && g_amg_fused;  // until a launch is refused in this solve
   constexpr int kFinePerIter = 5;  // level-0 SpMVs per iteration: S1, S2, S3, S4, q = A p
   while (c.done == kRun) {
     if (c.replace) {
@@ -4262,7 +4265,7 @@ int pcg_impl(fem_amg* h, const fem_matrix* A, const fem_operator64* op, const do
       }
       continue;
     }
-    if (!timing && g_amg_fused && launch_fused_cg<B0, K>(h, st)) {
+    if (fused && (fused = launch_fused_cg<B0, K>(h, st))) {
       rc = check_cuda("AMG CG");
       if (!rc) rc = read_ctrl(h, &c, st);
       if (rc) return rc;
