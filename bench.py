@@ -16,7 +16,7 @@ value      mixed precision: FP32 K and FP32 CG with FP64 residual
 e2e        the same through the public API from host tensors: the model is
            built from CPU tensors, so every step copies its inputs to the
            device and its results (u, f, sigma, F, grad) back.
-plain_fp64 the FP64 Jacobi-CG path (scalar CSR in the reference pattern).
+plain_fp64 the FP64 Jacobi-CG path (assembled in the reference's CSR pattern).
 mixed_block_jacobi  the mixed path with block Jacobi (the persistent CG
            kernel), reported beside the headline.
 
@@ -453,13 +453,25 @@ def heat_cpu_baseline(n_sample: int, n_target: int):
                         "cg_iterations": [it_s, it_l], "iteration_exponent": alpha, "predicted_seconds": t_t}}
 
 
-def timed_steps(lib, fn, steps, stream):
-    """Runs fn() `steps` times between CUDA events on `stream` with the
-    library's CG timing on; returns (ms per step, CG iterations per step,
-    summed CG unit time in ms, timed units, kernel launches, clock summary,
-    the last result)."""
+def unit_pass(lib, fn, steps=3):
+    """fn() `steps` times with the library's CG timing on, for the rooflines: summed unit
+    time in ms and timed units of the solve stats that fn returns.  Not for step times:
+    the timing puts events between launches, and sends multigrid systems that
+    otherwise run as one launch to the separate ones."""
     lib.fem_set_timing(1)
-    spmv_ms, spmv_n, iters, out = 0.0, 0, [], None
+    try:
+        stats = [fn() for _ in range(steps)]
+    finally:
+        lib.fem_set_timing(0)
+    return sum(s.spmv_ms for s in stats), sum(s.spmv_timed for s in stats)
+
+
+def timed_steps(lib, fn, steps, stream):
+    """Runs fn() `steps` times between CUDA events on `stream`, as a user's
+    program does, then a pass with the library's CG timing (unit_pass);
+    returns (ms per step, CG iterations per step, summed CG unit time in ms,
+    timed units, kernel launches, clock summary, the last result)."""
+    iters, out = [], None
     launches0 = lib.fem_launch_count()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     with ClockSampler(stream.device.index or 0) as clocks:
@@ -467,14 +479,11 @@ def timed_steps(lib, fn, steps, stream):
         ev0.record(stream)
         for _ in range(steps):
             out, model = fn()
-            st = model.last_solve
-            iters.append(st.iterations)
-            spmv_ms += st.system.stats.spmv_ms
-            spmv_n += st.system.stats.spmv_timed
+            iters.append(model.last_solve.iterations)
         ev1.record(stream)
         torch.cuda.synchronize()
     launches = lib.fem_launch_count() - launches0
-    lib.fem_set_timing(0)
+    spmv_ms, spmv_n = unit_pass(lib, lambda: fn()[1].last_solve.system.stats, min(steps, 3))
     return ev0.elapsed_time(ev1) / steps, iters, spmv_ms, spmv_n, launches, clocks.summary(), out
 
 
@@ -656,9 +665,7 @@ def run_assembly(args):
     for _ in range(max(args.warmup, 0)):
         assembly_step(asm, a, E0, point, args.stol)
     stream = torch.cuda.current_stream(dev)
-    lib.fem_set_timing(1)
     launches0 = lib.fem_launch_count()
-    spmv_ms = spmv_n = 0
     iters = []
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     with ClockSampler(0) as clocks:
@@ -666,14 +673,16 @@ def run_assembly(args):
         ev0.record(stream)
         for _ in range(args.steps):
             u, g = assembly_step(asm, a, E0, point, args.stol)
-            st = asm.last_solve
-            iters.append(st.iterations)
-            spmv_ms += st.spmv_ms
-            spmv_n += st.spmv_timed
+            iters.append(asm.last_solve.iterations)
         ev1.record(stream)
         torch.cuda.synchronize()
-    lib.fem_set_timing(0)
     launches = lib.fem_launch_count() - launches0
+
+    def unit_step():
+        assembly_step(asm, a, E0, point, args.stol)
+        return asm.last_solve
+
+    spmv_ms, spmv_n = unit_pass(lib, unit_step, 1)
     ms = ev0.elapsed_time(ev1) / args.steps
     st = asm.last_solve
     n_dofs = asm.n_dofs
@@ -997,8 +1006,7 @@ def main():
     for _ in range(max(args.warmup, 0)):
         out = step(m, forces, "mixed", args.stol, pc)
     torch.cuda.synchronize()
-    lib.fem_set_timing(1)
-    spmv_ms, spmv_n, iters = 0.0, 0, []
+    iters = []
     launches0 = lib.fem_launch_count()
     if dist is not None:
         dist.barrier()
@@ -1008,16 +1016,18 @@ def main():
         ev0.record(stream)
         for _ in range(args.steps):
             out = step(m, forces, "mixed", args.stol, pc)
-            st = m.last_solve
-            iters.append(st.iterations)
-            spmv_ms += st.system.stats.spmv_ms
-            spmv_n += st.system.stats.spmv_timed
+            iters.append(m.last_solve.iterations)
         ev1.record(stream)
         torch.cuda.synchronize()
     launches = lib.fem_launch_count() - launches0
-    lib.fem_set_timing(0)
     ms = ev0.elapsed_time(ev1) / args.steps
     ms = reduce_max(dist, ms, dev)
+
+    def unit_step():
+        step(m, forces, "mixed", args.stol, pc)
+        return m.last_solve.system.stats
+
+    spmv_ms, spmv_n = unit_pass(lib, unit_step, min(args.steps, 3))
     u_mixed, g_mixed = out[0], out[5]
 
     # end to end through the public API from host tensors
@@ -1125,8 +1135,8 @@ def main():
             "config": {"workload": f"hexa1_cube_{args.n}^3_jittered_linear_elastic_solve+adjoint",
                        "preconditioner": "smoothed-aggregation multigrid" if pc == "amg" else "block Jacobi",
                        "level0_smoothing": args.smoother if pc == "amg" else None,
-                       "fp64_residual": "FP64 copy of the sliced matrix" if args.residual == "copy"
-                       else "element pass",
+                       "fp64_residual": "element pass" if args.residual == "elements"
+                       else "FP64 copy of the sliced matrix",
                        "dofs": n_dofs, "nnz": dm.nnz, "n_elem": n_elem, "stol": args.stol,
                        "parallelism": "replicas" if world > 1 else "single",
                        "l2": "inputs larger than L2 (FP32 K = %.0f MB)" % (dm.n_blocks * 40 / 1e6)},
