@@ -3340,8 +3340,8 @@ struct fem_amg {
   // Memory that lives as long as the handle.  A hierarchy takes some 140 pieces, most
   // of them small, and a cudaMalloc costs 15 to 40 us and its cudaFree 10 to 30, so they
   // are cut from blocks; a block doubles the sum of the earlier ones, from 2 up
-  // to 64 MB, and no more than the last is left unused.  Pieces of 16 MB and more are
-  // allocated by themselves.  Create and destroy of the hierarchy of 27 x 22 x 31
+  // to 64 MB.  What an earlier block has left when a piece does not fit it stays
+  // unused, less than that piece.  Pieces of 16 MB and more are allocated by themselves.  Create and destroy of the hierarchy of 27 x 22 x 31
   // hexahedra, wall time: 4.0 and 1.0 ms by single pieces, 3.3 and 0.4 from blocks.
   template <typename T>
   T* alloc(int64_t count, cudaStream_t st) {

@@ -739,7 +739,6 @@ template <> struct DotAcc<double> {
   static constexpr bool kPlain = true;
   double v = 0.0;
   __device__ __forceinline__ void fma(double a, double b) { v = ::fma(a, b, v); }
-  __device__ __forceinline__ void shfl_down(int o) { v += __shfl_down_sync(0xffffffffu, v, o); }
   __device__ __forceinline__ double value() const { return v; }
 };
 // (round-to-nearest intrinsics: never contracted into an FMA)
