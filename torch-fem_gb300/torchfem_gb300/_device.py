@@ -588,14 +588,17 @@ class DeviceMesh:
         )
         return res, sumsq
 
-    # FP64 CG, CSR or sliced blocks.  CSR systems of up to CG_CLUSTER_NNZ[d] stored
-    # values run on the one-cluster kernel, about as fast there as the sliced
-    # grid-wide one (us an iteration, cluster / sliced: 10^3 cube, 268k values,
-    # 9.8 / 10.6; plane stress, 182k 7.7 / 8.1, 261k 9.3 / 8.2; 20^3 heat cube,
-    # 227k, 9.9 / 9.8) and ahead below.  Beyond, the sliced form is taken while its
-    # padding stores at most CG_SELL_PAD times the CSR values (Tetra1, 1.49 times:
-    # 19 against 33 us an iteration; the product's time grows with the stored slots,
-    # so at twice the values the gain would be gone).
+    # FP64 CG, CSR or sliced blocks.  Up to CG_CLUSTER_NNZ[d] stored values a system
+    # stays CSR, for the one-cluster kernel.  The bounds lie where that kernel and the
+    # sliced grid-wide one cross (us an iteration, cluster / sliced): Hexa1 198k values
+    # 8.2 / 9.5, 268k 8.9 / 9.7, 294k 10.4 / 9.9; Tetra1 230k 9.0 / 8.9; Tetra2 249k 12.1 /
+    # 15.8; Hexa2 267k 10.6 / 16.8; plane stress 178k 7.5 / 8.3, 232k 9.1 / 8.0; heat,
+    # Hexa1 195k 7.0 / 7.8, 262k 9.4 / 9.1.  What is below a bound but does not fit
+    # the cluster (16,384 rows, its shared memory: Quad1 heat from 16,100 nodes to 190k
+    # values) runs on the grid-wide CSR kernel, 12.9 to 14.4 us an iteration.  Beyond,
+    # the sliced form is taken while its padding stores at most CG_SELL_PAD times the
+    # CSR values (Tetra1, 1.49 times: 19 against 33 us an iteration; the product's time
+    # grows with the stored slots, so at twice the values the gain would be gone).
     CG_CLUSTER_NNZ = {1: 190_000, 2: 190_000, 3: 270_000}
     CG_SELL_PAD = 1.6
 
